@@ -23,6 +23,7 @@
 #include "fft_f32.cuh"
 #include "pbs_common.cuh"
 #include "ring.cuh"
+#include "split_steps.cuh"
 #include "tc_stage1.cuh"
 
 #include <type_traits>
@@ -48,77 +49,6 @@ struct Pbs01SplitSmem {
     static constexpr int TOTAL_TC = TC_SLOT_OFF + 16;
     static constexpr int TOTAL = WARP_OFF + W * PER_WARP;
 };
-
-// the decomposition words of (X^a - 1) * poly, once per polynomial:
-// w[2 m2 + h] = (((X^a - 1) poly)[m + 512 h] + offset + round) ^ DEC1_XOR,
-// m = lane + 32 m2; each of the l = 3 digits is then a field of these words
-__device__ __forceinline__ void digit_words1(uint32_t w[32], const uint32_t *poly, uint32_t abar, int lane)
-{
-#pragma unroll
-    for (int m2 = 0; m2 < 16; ++m2) {
-        const int m = lane + 32 * m2;
-        w[2 * m2] = ((rot_coef<N1>(poly, m, abar) - poly[m]) + DEC1_OFFSET + DEC1_ROUND) ^ DEC1_XOR;
-        w[2 * m2 + 1] = ((rot_coef<N1>(poly, m + 512, abar) - poly[m + 512]) + DEC1_OFFSET + DEC1_ROUND) ^ DEC1_XOR;
-    }
-}
-
-// v[m2] = (dig_d(m) + i dig_d(m+512)) * w^{32 m2} from the cached words: the
-// per-register part of the twist (ffft512_fwd_tw applies the lane's part)
-__device__ __forceinline__ void digits_from_words_f(float2 v[16], const uint32_t w[32], int d)
-{
-#pragma unroll
-    for (int m2 = 0; m2 < 16; ++m2) {
-        const int d0 = digit_field1(w[2 * m2], d), d1 = digit_field1(w[2 * m2 + 1], d);
-        v[m2] = cw64(make_float2((float)d0, (float)d1), m2);
-    }
-}
-
-// round(h) * 2^24 mod 2^32 without a conversion instruction: adding
-// 1.5 * 2^23 leaves round-to-nearest-even of h in the low mantissa bits
-// (|h| < 2^22, ~40 standard deviations of the hi products), and the term
-// needs only their low 8 bits.  Same bits as __float2int_rn(h) << 24, on the
-// FMA and ALU pipes instead of the conversion unit (measured: 1,024 PBS
-// 9.73 -> 9.41 ms, 1,184 in the 8-per-CTA shape 10.95 -> 10.5 ms; building
-// the digits from their bits the same way measured slower in both shapes, so
-// they keep the int -> float conversion)
-__device__ __forceinline__ uint32_t hi_term(float h)
-{
-    return __float_as_uint(h + 12582912.0f) << 24;
-}
-
-// poly[m] += round(hi_m) * 2^24 + round(lo_m) (mod 2^32), one read-modify-write
-// of the accumulator per polynomial.  f holds the hi and lo limbs of one
-// output as pairs, inverse-transformed together.  The hi limb's products
-// round exactly; the lo limb's FP32 error stays far below the bootstrapping
-// noise.
-__device__ __forceinline__ void add_inverse_split(uint32_t *poly, CP f[16], unsigned long long *xp, int lane,
-                                                  const Fft512TablesFold &T)
-{
-    pfft512_inv<true>(f, xp, T, lane);
-#pragma unroll
-    for (int m2 = 0; m2 < 16; ++m2) {
-        const int m = lane + 32 * m2;
-        const CP y = untwist_m2(f[m2], m2);
-        const float2 re = unpk2(y.re), im = unpk2(y.im);   // (hi, lo) of coefficients m and m + 512
-        poly[m] += hi_term(re.x) + (uint32_t)__float2ll_rn(re.y);
-        poly[m + 512] += hi_term(im.x) + (uint32_t)__float2ll_rn(im.y);
-    }
-}
-
-// f += v * k for both limbs of one output: k = (hi.re, lo.re, hi.im, lo.im),
-// vr = (v.re, v.re), vi = (v.im, v.im), nvi = (-v.im, -v.im)
-__device__ __forceinline__ void pmac(CP &f, unsigned long long vr, unsigned long long vi, unsigned long long nvi,
-                                     float4 k)
-{
-    const unsigned long long kr = pk2(k.x, k.y), ki = pk2(k.z, k.w);
-    f.re = f2(nvi, ki, f2(vr, kr, f.re));
-    f.im = f2(vi, kr, f2(vr, ki, f.im));
-}
-__device__ __forceinline__ CP pmul_first(unsigned long long vr, unsigned long long vi, unsigned long long nvi, float4 k)
-{
-    const unsigned long long kr = pk2(k.x, k.y), ki = pk2(k.z, k.w);
-    return CP{f2(nvi, ki, m2(vr, kr)), f2(vi, kr, m2(vr, ki))};
-}
 
 // Tensor-core stage 1 (tc_stage1.cuh), shared by the warps of a group of
 // four (warps 0-3 and 4-7; a producer warp takes no part), one polynomial at

@@ -72,6 +72,10 @@ struct Pbs01Args {
 cudaError_t launch_pbs01_f64(const Pbs01Args &a, int num_sms, int w, cudaStream_t st);
 // bk: split-precision key (float4 hi/lo chunk layout), tables: Fft512TablesF
 cudaError_t launch_pbs01_split(const Pbs01Args &a, int num_sms, int w, cudaStream_t st);
+// the same arithmetic, word for word, with 24 warps on one ciphertext per CTA
+// (pbs01_wide.cu)
+cudaError_t launch_pbs01_wide_f64(const Pbs01Args &a, int num_sms, cudaStream_t st);
+cudaError_t launch_pbs01_wide_split(const Pbs01Args &a, int num_sms, cudaStream_t st);
 // the same with the first step of every digit transform on the tensor cores
 cudaError_t launch_pbs01_split_tc(const Pbs01Args &a, int num_sms, int w, cudaStream_t st);
 
@@ -141,7 +145,72 @@ inline int pbs02_choose_p(int B, int num_sms, const float pass_ms[NSHAPES])
 {
     return choose_shape(B, num_sms, PBS02_SHAPES, pass_ms);
 }
+// How one call's batch is run: up to two launches, each in a shape of the
+// table (w ciphertexts per CTA) or, w = 1 on lvl01, by the kernel that has all
+// of an SM on one ciphertext.  Every kernel of a path gives the same words, so
+// this is a choice of time only:
+//   * the whole batch in the shape the table picks;
+//   * the whole batch with one ciphertext per SM at a time;
+//   * full passes of one shape, and the rest, which would be a mostly empty
+//     pass, by whichever of the others is shortest for it.
+// `one_ratio` is the measured time of a pass of one ciphertext per SM over
+// that of the shape `one_of`; the estimate scales with the context's table, and
+// a table that was never measured is replaced by the times of a B200
+// (`b200_ms`).
+struct BatchPart {
+    int n;   // ciphertexts
+    int w;   // per CTA
+};
+struct BatchPlan {
+    int parts;
+    BatchPart part[2];
+};
+struct ShapeTimes {
+    float b200_ms[NSHAPES];
+    int one_of;
+    float one_ratio;
+};
+// pass times (ms) on a B200 in the order of PBS01_SHAPES: 7, 8, 4 per CTA; one
+// ciphertext per SM 2.30 (split) and 3.18 (FP64) of the 4-per-CTA pass
+constexpr ShapeTimes PBS01_SPLIT_TIMES = {{9.40f, 10.31f, 7.50f}, 2, 0.307f};
+constexpr ShapeTimes PBS01_F64_TIMES = {{14.21f, 14.60f, 10.58f}, 2, 0.301f};
+
+inline BatchPlan plan_batch(int B, int num_sms, const int shapes[NSHAPES], const float pass_ms[NSHAPES],
+                            const ShapeTimes &times)
+{
+    const float *ms = shape_table_measured(pass_ms) ? pass_ms : times.b200_ms;
+    const float one_ms = times.one_ratio * ms[times.one_of];
+    auto passes = [&](int n, int w) { return (float)(((n + w - 1) / w + num_sms - 1) / num_sms); };
+    // the best single launch for n ciphertexts: ties to the table's shapes
+    auto single = [&](int n, int &w) {
+        const int s = choose_shape(n, num_sms, shapes, ms);
+        float cost = 0.0f;
+        for (int i = 0; i < NSHAPES; ++i)
+            if (shapes[i] == s) cost = passes(n, s) * ms[i];
+        w = s;
+        const float one = passes(n, 1) * one_ms;
+        if (one < cost) {
+            w = 1;
+            cost = one;
+        }
+        return cost;
+    };
+    BatchPlan best{1, {{B, 0}, {0, 0}}};
+    float best_cost = single(B, best.part[0].w);
+    for (int i = 0; i < NSHAPES; ++i) {
+        const int full = shapes[i] * num_sms, k = B / full, rest = B - k * full;
+        if (k == 0 || rest == 0) continue;
+        int w = 0;
+        const float cost = k * ms[i] + single(rest, w);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = BatchPlan{2, {{k * full, shapes[i]}, {rest, w}}};
+        }
+    }
+    return best;
+}
 cudaError_t init_pbs01_f64();
 cudaError_t init_pbs01_split();
+cudaError_t init_pbs01_wide();
 
 }  // namespace cfdb

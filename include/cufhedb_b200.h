@@ -391,10 +391,13 @@ CUFHEDB_API int cufhedb_selftest_wait_timeout(cufhedb_ctx *ctx, uint32_t polls);
  * takes ceil(ceil(B / shape) / SMs) passes; every launch (PBS, gates,
  * operator chains) picks the shape with the least passes x measured pass
  * time, ties to the earlier shape; without measurements all pass times count
- * as equal.  CUFHEDB_SPLIT32 launches also pick the layout of the first
- * transform step, on the CUDA cores or on the tensor cores (the
- * CUFHEDB_SPLIT32_TC kernel), by the same rule over both tables once both
- * are measured, ties to the CUDA cores.  No counterpart in the reference,
+ * as equal.  The lvl01 paths (not CUFHEDB_SPLIT32_TC) may divide a batch:
+ * a small batch, or what is left after a shape's full passes, runs on a
+ * kernel with one ciphertext per SM or in another shape where that is
+ * shorter; the results are the same words.  CUFHEDB_SPLIT32 launches also
+ * pick the layout of the first transform step, on the CUDA cores or on the
+ * tensor cores (the CUFHEDB_SPLIT32_TC kernel), by the same rule over both
+ * tables once both are measured, ties to the CUDA cores.  No counterpart in the reference,
  * which runs one ciphertext per launch.  The tuning calls are synchronous;
  * call them outside stream capture. */
 /* times one full pass of each lvl01 shape for `precision` (uniform random lvl0
@@ -406,7 +409,7 @@ CUFHEDB_API int cufhedb_autotune_pbs02(cufhedb_ctx *ctx, float *ms);
 /* the context's table for a level (1 with FP64 or SPLIT32, 2 with FP64):
  * shapes[3] and pass_ms[3] (either may be NULL); returns 3 */
 CUFHEDB_API int cufhedb_autotune_table(cufhedb_ctx *ctx, int level, int precision, int *shapes, float *pass_ms);
-/* the shape (ciphertexts per CTA) a launch of B ciphertexts would use now */
+/* the table's shape (ciphertexts per CTA) for a launch of all B ciphertexts */
 CUFHEDB_API int cufhedb_launch_shape(cufhedb_ctx *ctx, int level, int precision, int B, int *shape);
 /* the stage-1 layout a CUFHEDB_SPLIT32 launch of B ciphertexts would use now:
  * *tensor_core_stage1 = 1 (tensor cores) or 0 (CUDA cores) */
