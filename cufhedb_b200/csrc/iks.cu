@@ -97,7 +97,28 @@ __device__ __forceinline__ uint64_t iks_input(const IksArgs &a, size_t base, int
     }
 }
 
-template <int NT, bool WIDE, int NIN, int BASEBIT, int TT, int NOUT>
+// the output's b word before any key row: b' of the reference
+template <bool WIDE, int NIN>
+__device__ __forceinline__ uint32_t iks_b(const IksArgs &a, size_t base)
+{
+    if constexpr (WIDE) return (uint32_t)((a.in64[base + NIN] + a.offset64 + (1ull << 31)) >> 32);
+    else return (uint32_t)iks_input<false>(a, base, NIN) + a.offset;
+}
+
+// (0, ..., 0, b'): what the parts of a divided switch add to
+template <bool WIDE, int NIN, int NOUT>
+__global__ void iks_init_kernel(IksArgs a)
+{
+    const int ct = blockIdx.x;
+    const uint32_t b = iks_b<WIDE, NIN>(a, (size_t)ct * (NIN + 1));
+    for (int k = threadIdx.x; k < NOUT; k += blockDim.x) a.out[(size_t)ct * NOUT + k] = k == NOUT - 1 ? b : 0u;
+}
+
+// one CTA per (ciphertext, part of the input coefficients).  With one part
+// (PARTS false) it writes its ciphertext's output; otherwise every part adds
+// its sum to the initialised output (integer sums modulo 2^32: any order gives
+// the same words).
+template <int NT, bool WIDE, int NIN, int BASEBIT, int TT, int NOUT, bool PARTS>
 __global__ void __launch_bounds__(NT) iks_kernel(IksArgs a)
 {
     static_assert(NT % 32 == 0, "whole warps");
@@ -116,14 +137,16 @@ __global__ void __launch_bounds__(NT) iks_kernel(IksArgs a)
     for (int p = 0; p < PER; ++p) acc[p] = make_uint4(0u, 0u, 0u, 0u);
 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int i0 = 0; i0 < NIN; i0 += NT) {
+    const int first = PARTS ? (int)((long long)NIN * blockIdx.y / gridDim.y) : 0;
+    const int last = PARTS ? (int)((long long)NIN * (blockIdx.y + 1) / gridDim.y) : NIN;
+    for (int i0 = first; i0 < last; i0 += NT) {
         // the chunk's selected rows, compacted in key order (ascending i, j)
         // so that every CTA of the batch walks the key the same way and rows
         // that several ciphertexts select are fetched close together in time
         const int i = i0 + threadIdx.x;
         uint32_t ids[TT];
         int n = 0;
-        if (i < NIN) {
+        if (i < last) {
             const uint64_t abar = iks_input<WIDE>(a, base, i) + prec;
 #pragma unroll
             for (int j = 0; j < TT; ++j) {
@@ -154,20 +177,55 @@ __global__ void __launch_bounds__(NT) iks_kernel(IksArgs a)
         __syncthreads();
     }
 
-    uint32_t bnew;
-    if constexpr (WIDE) bnew = (uint32_t)((a.in64[base + NIN] + a.offset64 + (1ull << 31)) >> 32);
-    else bnew = (uint32_t)iks_input<false>(a, base, NIN) + a.offset;
     uint32_t *o = a.out + (size_t)ct * NOUT;
+    const uint32_t bnew = PARTS ? 0u : iks_b<WIDE, NIN>(a, base);
 #pragma unroll
     for (int p = 0; p < PER; ++p) {
         const int k0 = 4 * (threadIdx.x + p * NT);
         const uint32_t v[4] = {acc[p].x, acc[p].y, acc[p].z, acc[p].w};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            if (k0 + c < NOUT - 1) o[k0 + c] = v[c];
-            else if (k0 + c == NOUT - 1) o[k0 + c] = v[c] + bnew;
+            if (k0 + c >= NOUT) continue;
+            if constexpr (PARTS) atomicAdd(o + k0 + c, v[c]);
+            else o[k0 + c] = k0 + c == NOUT - 1 ? v[c] + bnew : v[c];
         }
     }
+}
+
+// Parts per ciphertext.  One CTA keeps 8 rows (24 KB) in flight and takes 0.57 ms
+// (lvl10) over its 2,048 rows however empty the GPU is, so a batch is divided
+// into about IKS_CTAS CTAs, of at least 16 input coefficients each; many short
+// CTAs also leave no half-empty last wave (IKS_WAVE of them are resident).
+// The undivided form is left where it is the faster one: a batch that nearly
+// fills one wave, or several, walks the key in step and shares its rows in L2.
+// Measured, ms undivided -> divided (lvl10 / lvl20 / lvl21):
+//   1: 0.213 -> 0.025 / 0.395 -> 0.026 / 3.42 -> 0.037
+//   148: 0.574 -> 0.142 / 1.08 -> 0.262 / 2.55 -> 0.58
+//   592: 0.589 -> 0.396 / 1.11 -> 0.768 / 2.29 -> 2.23
+//   700: 0.597 -> 0.489 / 1.14 -> 0.977;  1,024: 0.602 -> 0.663 / 1.20 -> 1.48
+//   1,500: 1.25 -> 0.957 / 2.31 -> 1.95;  2,048: 1.25 -> 1.29 / 2.38 -> 2.74
+constexpr int IKS_CTAS = 9472, IKS_WAVE = 1184;
+template <int NIN>
+int iks_parts(int B)
+{
+    if ((B > 850 && B <= IKS_WAVE) || B > 1900) return 1;
+    const int p = (IKS_CTAS + B - 1) / B;
+    return p < NIN / 16 ? p : NIN / 16;
+}
+
+template <int NT, bool WIDE, int NIN, int BASEBIT, int TT, int NOUT>
+cudaError_t launch_gather(const IksArgs &a, cudaStream_t st)
+{
+    const int parts = iks_parts<NIN>(a.B);
+    if (parts == 1) {
+        iks_kernel<NT, WIDE, NIN, BASEBIT, TT, NOUT, false><<<a.B, NT, 0, st>>>(a);
+        return cudaGetLastError();
+    }
+    iks_init_kernel<WIDE, NIN, NOUT><<<a.B, 256, 0, st>>>(a);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    iks_kernel<NT, WIDE, NIN, BASEBIT, TT, NOUT, true><<<dim3(a.B, parts), NT, 0, st>>>(a);
+    return cudaGetLastError();
 }
 
 // ---- key-stationary lvl2 -> lvl1 switch (large batches) ------------------------
@@ -314,15 +372,10 @@ cudaError_t launch_iks(const IksArgs &a, int kind, cudaStream_t st)
     }
     // one 16-byte word of a padded row per thread: 169 of 192 (lvl0 rows),
     // 257 of 288 (lvl1 rows)
-    if (kind == 10)
-        iks_kernel<192, false, N1, KS10_BASEBIT, KS10_T, N0 + 1><<<a.B, 192, 0, st>>>(a);
-    else if (kind == 20)
-        iks_kernel<192, true, N2, KS20_BASEBIT, KS20_T, N0 + 1><<<a.B, 192, 0, st>>>(a);
-    else if (kind == 21)
-        iks_kernel<288, true, N2, KS21_BASEBIT, KS21_T, N1 + 1><<<a.B, 288, 0, st>>>(a);
-    else
-        return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    if (kind == 10) return launch_gather<192, false, N1, KS10_BASEBIT, KS10_T, N0 + 1>(a, st);
+    if (kind == 20) return launch_gather<192, true, N2, KS20_BASEBIT, KS20_T, N0 + 1>(a, st);
+    if (kind == 21) return launch_gather<288, true, N2, KS21_BASEBIT, KS21_T, N1 + 1>(a, st);
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace cfdb
