@@ -203,6 +203,20 @@ int launch_pbs01_any(cufhedb_ctx *ctx, Pbs01Args &a, int precision, cudaStream_t
     return CUFHEDB_OK;
 }
 
+// the lvl02 PBS, divided over launches as the context's table makes shortest
+int launch_pbs02_any(cufhedb_ctx *ctx, const Pbs02Args &a, cudaStream_t st)
+{
+    const BatchPlan plan = plan_batch(a.B, ctx->num_sms, PBS02_SHAPES, ctx->pbs02_pass_ms, PBS02_TIMES);
+    Pbs02Args p = a;
+    for (int k = 0; k < plan.parts; ++k) {
+        p.B = plan.part[k].n;
+        CK(launch_pbs02_f64(p, ctx->num_sms, plan.part[k].w, st));
+        p.in += (size_t)p.B * (N0 + 1);
+        p.out += (size_t)p.B * (N2 + 1);
+    }
+    return CUFHEDB_OK;
+}
+
 int pbs01_enqueue(cufhedb_ctx *ctx, const uint32_t *in, uint32_t *out, int B, const cufhedb_testvec *tv,
                   int precision, cudaStream_t st)
 {
@@ -283,8 +297,7 @@ int pbs02_run(cufhedb_ctx *ctx, const uint32_t *in, uint64_t *out, int B, const 
     a.tv = tv;
     a.out_b_add = b_add;
     a.err = ctx->err;
-    CK(launch_pbs02_f64(a, ctx->num_sms, pbs02_choose_p(B, ctx->num_sms, ctx->pbs02_pass_ms), st));
-    return CUFHEDB_OK;
+    return launch_pbs02_any(ctx, a, st);
 }
 
 int iks_run(cufhedb_ctx *ctx, int kind, const void *in, const uint32_t *in_b, int sa, int sb, uint64_t offset,
@@ -1244,8 +1257,7 @@ static int pbs02_enqueue(cufhedb_ctx *ctx, const uint32_t *in, uint64_t *out, in
     a.tables = ctx->tab1024;
     a.tv = to_tv(tv);
     a.err = ctx->err;
-    CK(launch_pbs02_f64(a, ctx->num_sms, pbs02_choose_p(B, ctx->num_sms, ctx->pbs02_pass_ms), st));
-    return CUFHEDB_OK;
+    return launch_pbs02_any(ctx, a, st);
 }
 
 int cufhedb_pbs_lvl02(cufhedb_ctx *ctx, const uint32_t *in_lvl0, uint64_t *out_lvl2, int B, const cufhedb_testvec *tv,

@@ -247,8 +247,10 @@ __device__ __forceinline__ int fft8x_xp(int t, int k)
 // forward: v[j] = z_{t + T j} / w^t in (the inputs multiplied by W_32^j only),
 // v[s] = V(fft8x_freq<T>(t, s)) out.  xp: FFT8X_XP<T>-entry scratch shared
 // by the group; bar: its named barrier.
-template <typename C, int T>
-__device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Fft8xTables<C, T> &tab, int t, int bar)
+// after_first() runs in every thread past the first group barrier.
+template <typename C, int T, class Hook>
+__device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Fft8xTables<C, T> &tab, int t, int bar,
+                                          Hook after_first)
 {
     constexpr int L = T / 8;
     cx_dft8<1>(v);
@@ -257,6 +259,7 @@ __device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Fft8xTables<C, T>
 #pragma unroll
     for (int k = 0; k < 8; ++k) xp[fft8x_xp<C>(t, k)] = v[k];
     group_sync<T>(bar);
+    after_first();
     const int a = t % L, k = t / L;
 #pragma unroll
     for (int b = 0; b < 8; ++b) v[b] = xp[fft8x_xp<C>(a + L * b, k)];
@@ -282,6 +285,12 @@ __device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Fft8xTables<C, T>
         v[rl] = cx_add(p, q);
         v[rl + 4] = cx_sub(p, q);
     }
+}
+
+template <typename C, int T>
+__device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Fft8xTables<C, T> &tab, int t, int bar)
+{
+    fft8x_fwd<C, T>(v, xp, tab, t, bar, [] {});
 }
 
 // inverse: v[s] = V(fft8x_freq<T>(t, s)) in, v[j] = M z_{t + T j} / w^t out

@@ -1,0 +1,365 @@
+// Batched lvl0 -> lvl2 programmable bootstrapping (GateBootstrappingTLWE2TLWEFFT
+// <lvl02param>, thirdparty/TFHEpp/src/gatebootstrapping.cpp:14-23, BlindRotate
+// at include/gatebootstrapping.hpp:15-43 with domain lvl0, target lvl2: bbar =
+// 2N - (b >> 20), abar_i = (a_i + 2^19) >> 20).
+//
+// One persistent CTA per SM holds C = 1 or 2 ciphertexts and four teams of 128
+// threads (8 of the 1,024 points each, fft8x.cuh), 16 warps in all; the teams of
+// a ciphertext (4 or 2) divide every CMux:
+//   words     the decomposition words of both polynomials, half a polynomial
+//             or a whole one per team;
+//   transform in rounds (2 of 4 rows, or 4 of 2 rows), each team transforms one
+//             digit polynomial;
+//   products  a team takes its share of the frequency slots (2 or 4 of 8) of
+//             the round's rows into both outputs' accumulators, in registers;
+//   inverse   one team per output.
+// Thread u of every team sits in the same lane of the same SM sub-partition
+// (four warps per team), so words, spectra and accumulators pass between teams
+// through tensor memory (tmem_exchange.cuh) and shared memory keeps only the
+// accumulators, the transposes and the key.  With C = 2 the two ciphertexts
+// share nothing but the key stage, so one's transforms run under the other's
+// products and conversions.
+//
+// What bounds it: per ciphertext and CMux about 10,300 shared-memory wavefronts
+// (half of them the two transposes of each transform), 8,000 FP64-pipe cycles
+// and 8,000 issue slots per scheduler; at C = 2 the wavefronts run at 65 % of
+// their rate and FP64 at 49 %, the rest is the barriers and the latency between
+// the stages.  Pass times on a B200 (148 SMs): C = 1 6.20 ms, C = 2 10.89 ms,
+// where one team per ciphertext with both accumulators in its registers took
+// 10.26, 13.80 and, with three ciphertexts, 17.65 ms (the shape-3 launch here,
+// passes of two and of one: 17.1 ms).  On the way: all teams of both
+// ciphertexts in lock step 12.28 ms; key chunks released by 16 warps with an
+// atomic each 8.49 ms at C = 1, by a producer warp (which costs the others
+// their registers) 7.06 ms; one release per team and round 6.20 ms.
+#include "lvl2_steps.cuh"
+#include "ring.cuh"
+#include "tc_stage1.cuh"
+#include "tmem_exchange.cuh"
+
+namespace cfdb {
+
+namespace {
+
+constexpr int TEAMS = 4;
+
+// C ciphertexts per CTA, TPC teams each: a round is TPC rows of each
+// ciphertext (both outputs' chunks), SL frequency slots per thread in the
+// products
+template <int C>
+struct TeamShape {
+    static constexpr int TPC = TEAMS / C;
+    static constexpr int ROUNDS = 2 * L2 / TPC;
+    static constexpr int SL = 8 / TPC;
+    static constexpr int CHUNK = 16384;                 // one (row, output): 1024 complex
+    static constexpr int CHUNKS = 2 * TPC;              // per round
+    static constexpr int STAGED = C == 1 ? 7 : 4;       // of them in shared memory, the rest from global memory
+    static constexpr uint32_t BYTES = STAGED * CHUNK;
+    static constexpr int KEY_OFF = 128;
+    static constexpr int TAB_OFF = KEY_OFF + (int)BYTES;
+    static constexpr int XP_OFF = TAB_OFF + ((int)sizeof(Fft1024Tables) + 127) / 128 * 128;
+    static constexpr int XP_BYTES = FFT8X_XP<T2> * 16;
+    static constexpr int ACC_OFF = XP_OFF + TEAMS * XP_BYTES;
+    static constexpr int ACC_BYTES = 2 * N2 * 8;
+    static constexpr int TOTAL = ACC_OFF + C * ACC_BYTES;
+    static_assert(TOTAL <= 227 * 1024, "shared memory budget");
+};
+
+// The key of one round in shared memory: one bulk copy, issued by the last
+// team to release the round before.  Waits are bounded; after one gives up
+// nothing is waited for or issued any more.
+template <int C>
+struct RoundKey {
+    using S = TeamShape<C>;
+    unsigned char *head;    // mbarrier, release count, issue count, abort flag
+    unsigned char *stage;
+    const unsigned char *src;
+    uint32_t total;         // rounds this block consumes
+
+    __device__ __forceinline__ uint64_t *full() const { return reinterpret_cast<uint64_t *>(head); }
+    __device__ __forceinline__ int *count() const { return reinterpret_cast<int *>(head + 8); }
+    __device__ __forceinline__ int *issued() const { return reinterpret_cast<int *>(head + 12); }
+    __device__ __forceinline__ volatile int *abort_flag() const { return reinterpret_cast<volatile int *>(head + 16); }
+
+    __device__ __forceinline__ void init()
+    {
+        mbar_init(full(), 1);
+        *count() = 0;
+        *issued() = 0;
+        *abort_flag() = 0;
+        fence_barrier_init();
+    }
+    __device__ __forceinline__ void issue(uint32_t n)
+    {
+        ++*issued();
+        mbar_arrive_expect_tx(full(), S::BYTES);
+        bulk_g2s(stage, src + (size_t)(n % (N0 * S::ROUNDS)) * S::CHUNKS * S::CHUNK, S::BYTES, full());
+    }
+    __device__ __forceinline__ void acquire(uint32_t n, int *err)
+    {
+        if (*abort_flag() == 0 && !mbar_wait(full(), n & 1)) {
+            report_error(err, DEV_TIMEOUT_FULL);
+            *abort_flag() = 1;
+        }
+    }
+    // one thread per team, after the team's last read of round n
+    __device__ __forceinline__ void release(uint32_t n)
+    {
+        if (ring_release(count(), n, TEAMS) && n + 1 < total && *abort_flag() == 0) {
+            fence_proxy_async_smem();
+            issue(n + 1);
+        }
+    }
+    // one thread, at the end: nothing may still be landing
+    __device__ __forceinline__ void drain(int *err)
+    {
+        if (*abort_flag() != 0 && *issued() > 0 && !mbar_wait(full(), (uint32_t)(*issued() - 1) & 1))
+            report_error(err, DEV_TIMEOUT_DRAIN);
+    }
+};
+
+// tensor-memory columns (of every lane; a double is two columns)
+constexpr uint32_t TT_SPEC = 0;      // [round parity 2][team 4][slot 8][re im]
+constexpr uint32_t TT_WORDS = 256;   // [ciphertext][polynomial 2][16 words]
+constexpr uint32_t TT_ACC = 384;     // [ciphertext][output 2][slot 8][re im]
+
+__device__ __forceinline__ void put_c(uint32_t *x, double2 z)
+{
+    x[0] = (uint32_t)__double2loint(z.x);
+    x[1] = (uint32_t)__double2hiint(z.x);
+    x[2] = (uint32_t)__double2loint(z.y);
+    x[3] = (uint32_t)__double2hiint(z.y);
+}
+__device__ __forceinline__ double2 get_c(const uint32_t *x)
+{
+    return make_double2(__hiloint2double((int)x[1], (int)x[0]), __hiloint2double((int)x[3], (int)x[2]));
+}
+
+// the teams of a ciphertext meet; tensor-memory stores before it (waited for)
+// are visible to loads after it
+template <int C>
+__device__ __forceinline__ void ct_sync(int q)
+{
+    tc_fence_before();
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + TEAMS + q), "n"(TEAMS * T2 / C) : "memory");
+    tc_fence_after();
+}
+
+template <int C>
+__global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
+{
+    using S = TeamShape<C>;
+    constexpr int TPC = S::TPC, SL = S::SL, ROUNDS = S::ROUNDS;
+    extern __shared__ __align__(128) unsigned char smem[];
+    Fft1024Tables *T = reinterpret_cast<Fft1024Tables *>(smem + S::TAB_OFF);
+    const int ngroups = (a.B + C - 1) / C;
+    RoundKey<C> key{smem, smem + S::KEY_OFF, reinterpret_cast<const unsigned char *>(a.bk),
+                    (uint32_t)groups_of_block(ngroups, blockIdx.x, gridDim.x) * N0 * ROUNDS};
+    uint32_t *slot = reinterpret_cast<uint32_t *>(smem + 64);
+
+    const int warp = threadIdx.x >> 5;
+    const int team = threadIdx.x / T2, t = threadIdx.x % T2, bar = 1 + team;
+    const int q = team / TPC, h = team % TPC;   // the ciphertext, and the team's place in it
+    if (threadIdx.x == 0) key.init();
+    if (warp == 0) tmem_alloc(slot, 512);
+    {
+        const double2 *src = reinterpret_cast<const double2 *>(a.tables);
+        double2 *dst = reinterpret_cast<double2 *>(T);
+        for (int i = threadIdx.x; i < (int)(sizeof(Fft1024Tables) / 16); i += blockDim.x) dst[i] = src[i];
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (threadIdx.x == 0) key.issue(0);
+    const uint32_t tm = *slot + ((32u * (warp & 3)) << 16);
+
+    double2 *xp = reinterpret_cast<double2 *>(smem + S::XP_OFF + team * S::XP_BYTES);
+    uint64_t *acc = reinterpret_cast<uint64_t *>(smem + S::ACC_OFF + q * S::ACC_BYTES);
+
+    uint32_t n = 0;   // running number of the round
+    for (int g = blockIdx.x; g < ngroups; g += gridDim.x) {
+        const int ct = g * C + q;
+        const bool valid = ct < a.B;
+        const uint32_t *in = a.in + (size_t)(valid ? ct : 0) * (N0 + 1);
+        uint32_t an = in[0];   // the next CMux's mask word, read one CMux ahead
+        if (h == 0) {
+            for (int m = t; m < N2; m += T2) acc[m] = 0;
+        } else if (h == 1) {
+            const uint32_t bbar = 2 * N2 - (in[N0] >> 20);
+            for (int m = t; m < N2; m += T2) acc[N2 + m] = testvec_rot2(a.tv, m, bbar);
+        }
+        ct_sync<C>(q);
+
+        for (int i = 0; i < N0; ++i) {
+            const uint32_t ab = valid ? (an + (1u << 19)) >> 20 : 0u;
+            an = in[i + 1];
+            if (ab == 0) {
+                for (int k = 0; k < ROUNDS; ++k, ++n) {
+                    key.acquire(n, a.err);
+                    if (t == 0) key.release(n);
+                }
+                continue;
+            }
+            {
+                // the decomposition words of polynomial h % 2: all 16 with two
+                // teams per ciphertext, one half of them with four
+                constexpr int NW = C == 2 ? 8 : 4;
+                const int j0 = C == 2 ? 0 : 4 * (h >> 1);
+                const uint64_t *poly = acc + (h & 1) * N2;
+                uint32_t x[4 * NW];
+#pragma unroll
+                for (int j = 0; j < NW; ++j) {
+                    uint64_t w0, w1;
+                    digit_word_pair2<true>(w0, w1, poly, ab, t + T2 * (j0 + j));
+                    x[4 * j] = (uint32_t)w0;
+                    x[4 * j + 1] = (uint32_t)(w0 >> 32);
+                    x[4 * j + 2] = (uint32_t)w1;
+                    x[4 * j + 3] = (uint32_t)(w1 >> 32);
+                }
+                const uint32_t col = tm + TT_WORDS + 64 * q + 32 * (h & 1);
+                if constexpr (C == 2) tmem_st32_nowait(col, x);
+                else tmem_st16_nowait(col + 4 * j0, x);
+                tmem_wait_st();
+            }
+            ct_sync<C>(q);
+            double2 f[2][SL];   // [output][slot SL h + s]
+#pragma unroll 1
+            for (int k = 0; k < ROUNDS; ++k, ++n) {
+                {
+                    const int r = TPC * k + h;
+                    uint32_t x[32];
+                    tmem_ld32_nowait(tm + TT_WORDS + 64 * q + 32 * (r / L2), x);
+                    tmem_wait_ld();
+                    tmem_landed<32>(x);
+                    uint64_t w[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) w[j] = ((uint64_t)x[2 * j + 1] << 32) | x[2 * j];
+                    double2 v[8];
+                    digits2(v, w, r % L2);
+                    // every thread of the team is past its products of the
+                    // round before when it reaches the transform's first barrier
+                    fft8x_fwd<double2, T2>(v, xp, *T, t, bar, [&] {
+                        if (k > 0 && t == 0) key.release(n - 1);
+                    });
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) put_c(x + 4 * s, v[s]);
+                    tmem_st32_nowait(tm + TT_SPEC + 128 * (k & 1) + 32 * team, x);
+                    tmem_wait_st();
+                }
+                ct_sync<C>(q);
+                // chunk e of the round: row TPC k + e / 2, output e % 2; this
+                // thread's values at [slot][t]
+                const float4 *kg = reinterpret_cast<const float4 *>(a.bk) +
+                                   ((size_t)(i * ROUNDS + k) * S::CHUNKS) * 1024 + SL * h * T2 + t;
+                float4 far[S::CHUNKS - S::STAGED + 1][SL];
+#pragma unroll
+                for (int e = S::STAGED; e < S::CHUNKS; ++e)
+#pragma unroll
+                    for (int s = 0; s < SL; ++s) far[e - S::STAGED][s] = __ldg(kg + e * 1024 + s * T2);
+                key.acquire(n, a.err);
+                const double2 *ks = reinterpret_cast<const double2 *>(smem + S::KEY_OFF) + SL * h * T2 + t;
+#pragma unroll
+                for (int rr = 0; rr < TPC; ++rr) {
+                    uint32_t y[4 * SL];
+                    const uint32_t col = tm + TT_SPEC + 128 * (k & 1) + 32 * (TPC * q + rr) + 4 * SL * h;
+                    if constexpr (SL == 4) tmem_ld16_nowait(col, y);
+                    else tmem_ld8_nowait(col, y);
+                    tmem_wait_ld();
+                    tmem_landed<4 * SL>(y);
+#pragma unroll
+                    for (int o = 0; o < 2; ++o) {
+                        const int e = 2 * rr + o;
+#pragma unroll
+                        for (int s = 0; s < SL; ++s) {
+                            const double2 kv = e < S::STAGED ? ks[e * 1024 + s * T2]
+                                                             : *reinterpret_cast<const double2 *>(&far[e - S::STAGED][s]);
+                            const double2 v = get_c(y + 4 * s);
+                            if (k == 0 && rr == 0) f[o][s] = cx_mul(v, kv);
+                            else cx_fma(f[o][s], v, kv);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                uint32_t x[4 * SL];
+#pragma unroll
+                for (int s = 0; s < SL; ++s) put_c(x + 4 * s, f[o][s]);
+                const uint32_t col = tm + TT_ACC + 64 * q + 32 * o + 4 * SL * h;
+                if constexpr (SL == 4) tmem_st16_nowait(col, x);
+                else tmem_st8_nowait(col, x);
+            }
+            tmem_wait_st();
+            ct_sync<C>(q);
+            if (t == 0) key.release(n - 1);
+            if (h < 2) {
+                uint32_t x[32];
+                tmem_ld32_nowait(tm + TT_ACC + 64 * q + 32 * h, x);
+                tmem_wait_ld();
+                tmem_landed<32>(x);
+                double2 v[8];
+#pragma unroll
+                for (int s = 0; s < 8; ++s) v[s] = get_c(x + 4 * s);
+                fft8x_inv<double2, T2>(v, xp, *T, t, bar);
+                add_inverse2(acc + h * N2, v, t);
+            }
+            ct_sync<C>(q);
+        }
+        if (valid) {
+            uint64_t *o = a.out + (size_t)ct * (N2 + 1);
+            for (int m = t + h * T2; m < N2; m += TPC * T2) o[m] = m == 0 ? acc[0] : 0ull - acc[N2 - m];
+            if (h == 0 && t == 0) o[N2] = acc[N2] + a.out_b_add;
+        }
+        ct_sync<C>(q);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0) key.drain(a.err);
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(*slot, 512);
+    }
+}
+
+template <int C>
+cudaError_t launch_team_t(const Pbs02Args &a, int num_sms, cudaStream_t st)
+{
+    const int groups = (a.B + C - 1) / C;
+    pbs02_team_kernel<C><<<groups < num_sms ? groups : num_sms, TEAMS * T2, TeamShape<C>::TOTAL, st>>>(a);
+    return cudaGetLastError();
+}
+
+template <int C>
+cudaError_t init_team_t()
+{
+    return cudaFuncSetAttribute(pbs02_team_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                TeamShape<C>::TOTAL);
+}
+
+}  // namespace
+
+// p: ciphertexts per SM in a pass.  Three run as passes of two for two thirds
+// of the batch, then passes of one.
+cudaError_t launch_pbs02_f64(const Pbs02Args &a, int num_sms, int p, cudaStream_t st)
+{
+    if (a.B <= 0) return cudaSuccess;
+    if (p == 1) return launch_team_t<1>(a, num_sms, st);
+    if (p == 2) return launch_team_t<2>(a, num_sms, st);
+    if (p != 3) return cudaErrorInvalidValue;
+    const int passes = (a.B + 3 * num_sms - 1) / (3 * num_sms), two = 2 * num_sms * passes;
+    Pbs02Args r = a;
+    r.B = a.B < two ? a.B : two;
+    cudaError_t e = launch_team_t<2>(r, num_sms, st);
+    if (e != cudaSuccess || r.B == a.B) return e;
+    r.in += (size_t)r.B * (N0 + 1);
+    r.out += (size_t)r.B * (N2 + 1);
+    r.B = a.B - r.B;
+    return launch_team_t<1>(r, num_sms, st);
+}
+
+cudaError_t init_pbs02_f64()
+{
+    const cudaError_t e = init_team_t<1>();
+    return e == cudaSuccess ? init_team_t<2>() : e;
+}
+
+}  // namespace cfdb

@@ -82,7 +82,7 @@ cudaError_t launch_pbs01_split_tc(const Pbs01Args &a, int num_sms, int w, cudaSt
 // Launch shapes of the persistent PBS kernels, as ciphertexts per CTA: lvl01
 // 7 (with a producer warp on the split path), 8 and 4 (one warp per SM
 // sub-partition: the shortest pass, for batches that leave SMs idle); lvl02
-// 3, 2 and 1 (four warps per ciphertext).  Each CTA works through
+// 3 (passes of 2, then of 1), 2 and 1.  Each CTA works through
 // ceil(ceil(B / w) / SMs) passes of w ciphertexts; the autotuner measures
 // one full pass of every shape, and a launch takes the shape with the least
 // passes x pass time.  Ties go to the earlier shape in the list, so with no
@@ -174,6 +174,9 @@ struct ShapeTimes {
 // ciphertext per SM 2.30 (split) and 3.18 (FP64) of the 4-per-CTA pass
 constexpr ShapeTimes PBS01_SPLIT_TIMES = {{9.40f, 10.31f, 7.50f}, 2, 0.307f};
 constexpr ShapeTimes PBS01_F64_TIMES = {{14.21f, 14.60f, 10.58f}, 2, 0.301f};
+
+// lvl02: 3, 2 and 1 ciphertexts per SM (the last is the table's own shape 1)
+constexpr ShapeTimes PBS02_TIMES = {{17.15f, 10.89f, 6.20f}, 2, 1.0f};
 
 inline BatchPlan plan_batch(int B, int num_sms, const int shapes[NSHAPES], const float pass_ms[NSHAPES],
                             const ShapeTimes &times)
