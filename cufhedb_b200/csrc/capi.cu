@@ -160,13 +160,11 @@ int check_tv(const cufhedb_testvec *tv, int N)
 
 bool valid_precision(int p) { return p == CUFHEDB_FP64 || p == CUFHEDB_SPLIT32 || p == CUFHEDB_SPLIT32_TC; }
 
-// the lvl01 PBS of a precision, divided over kernels and launch shapes as the
-// context's table makes shortest (key, tables and kernel set in `a` here)
+// the lvl01 PBS kernel of a precision (key, tables and kernel set in `a` here)
 int launch_pbs01_any(cufhedb_ctx *ctx, Pbs01Args &a, int precision, cudaStream_t st)
 {
     // CUFHEDB_SPLIT32 lets the measured tables pick the stage-1 layout too;
-    // CUFHEDB_SPLIT32_TC forces the tensor-core one, whose words differ, so
-    // such a batch is never divided
+    // CUFHEDB_SPLIT32_TC forces the tensor-core one
     int w = pbs01_choose_w(a.B, ctx->num_sms, ctx->pbs01_pass_ms[precision]);
     if (precision == CUFHEDB_SPLIT32) {
         const SplitLaunch c = pbs01_split_choose(a.B, ctx->num_sms, ctx->pbs01_pass_ms[CUFHEDB_SPLIT32],
@@ -177,36 +175,21 @@ int launch_pbs01_any(cufhedb_ctx *ctx, Pbs01Args &a, int precision, cudaStream_t
     if (precision == CUFHEDB_FP64) {
         a.bk = ctx->bk01;
         a.tables = ctx->tab512;
-    } else {
-        if (!ctx->bk01_split) return fail(CUFHEDB_ERR_NOKEY, "split-precision lvl01 key not prepared");
-        a.bk = reinterpret_cast<const double2 *>(ctx->bk01_split);
-        a.tables = ctx->tab512f;
-    }
-    if (precision == CUFHEDB_SPLIT32_TC) {
-        CK(launch_pbs01_split_tc(a, ctx->num_sms, w, st));
+        CK(launch_pbs01_f64(a, ctx->num_sms, st));
         return CUFHEDB_OK;
     }
-    const bool f64 = precision == CUFHEDB_FP64;
-    const BatchPlan plan = plan_batch(a.B, ctx->num_sms, PBS01_SHAPES, ctx->pbs01_pass_ms[precision],
-                                      f64 ? PBS01_F64_TIMES : PBS01_SPLIT_TIMES);
-    Pbs01Args p = a;
-    for (int k = 0; k < plan.parts; ++k) {
-        p.B = plan.part[k].n;
-        if (plan.part[k].w == 1)
-            CK(f64 ? launch_pbs01_wide_f64(p, ctx->num_sms, st) : launch_pbs01_wide_split(p, ctx->num_sms, st));
-        else
-            CK(f64 ? launch_pbs01_f64(p, ctx->num_sms, plan.part[k].w, st)
-                   : launch_pbs01_split(p, ctx->num_sms, plan.part[k].w, st));
-        p.in += (size_t)p.B * (N0 + 1);
-        p.out += (size_t)p.B * (N1 + 1);
-    }
+    if (!ctx->bk01_split) return fail(CUFHEDB_ERR_NOKEY, "split-precision lvl01 key not prepared");
+    a.bk = reinterpret_cast<const double2 *>(ctx->bk01_split);
+    a.tables = ctx->tab512f;
+    if (precision == CUFHEDB_SPLIT32_TC) CK(launch_pbs01_split_tc(a, ctx->num_sms, w, st));
+    else CK(launch_pbs01_split(a, ctx->num_sms, st));
     return CUFHEDB_OK;
 }
 
 // the lvl02 PBS, divided over launches as the context's table makes shortest
 int launch_pbs02_any(cufhedb_ctx *ctx, const Pbs02Args &a, cudaStream_t st)
 {
-    const BatchPlan plan = plan_batch(a.B, ctx->num_sms, PBS02_SHAPES, ctx->pbs02_pass_ms, PBS02_TIMES);
+    const BatchPlan plan = plan_batch(a.B, ctx->num_sms, PBS02_SHAPES, ctx->pbs02_pass_ms, PBS02_B200_MS);
     Pbs02Args p = a;
     for (int k = 0; k < plan.parts; ++k) {
         p.B = plan.part[k].n;
@@ -390,9 +373,8 @@ int cufhedb_ctx_create(cufhedb_ctx **out, int device)
     if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(ctx->err, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->io, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = init_pbs01_f64();
-    if (e == cudaSuccess) e = init_pbs01_split();
-    if (e == cudaSuccess) e = init_pbs01_wide();
+    if (e == cudaSuccess) e = init_pbs01_ct();
+    if (e == cudaSuccess) e = init_pbs01_split_tc();
     if (e == cudaSuccess) e = init_pbs02_f64();
     if (e == cudaSuccess) e = init_extprod1();
     if (e == cudaSuccess) e = noalloc_scratch_address(&ctx->noalloc_scratch);
@@ -933,12 +915,12 @@ static int autotune_level(cufhedb_ctx *ctx, int level, int precision, float out_
                     if (precision == CUFHEDB_FP64) {
                         a.bk = ctx->bk01;
                         a.tables = ctx->tab512;
-                        e = launch_pbs01_f64(a, ctx->num_sms, w, st);
+                        e = launch_pbs01_f64(a, ctx->num_sms, st);
                     } else {
                         a.bk = reinterpret_cast<const double2 *>(ctx->bk01_split);
                         a.tables = ctx->tab512f;
                         e = precision == CUFHEDB_SPLIT32_TC ? launch_pbs01_split_tc(a, ctx->num_sms, w, st)
-                                                            : launch_pbs01_split(a, ctx->num_sms, w, st);
+                                                            : launch_pbs01_split(a, ctx->num_sms, st);
                     }
                 } else {
                     const cufhedb_testvec tv{CUFHEDB_TV_CONST, 0, 1ull << 61, nullptr};

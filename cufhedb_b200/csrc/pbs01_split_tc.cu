@@ -1,25 +1,9 @@
-// Batched lvl0 -> lvl1 programmable bootstrapping, split-precision FP32 path.
-//
-// Same algorithm as pbs01_f64.cu (TFHEpp GateBootstrappingTLWE2TLWEFFT
-// <lvl01param>, src/gatebootstrapping.cpp:14-23), with every transform and
-// product in FP32.  Precision plan (the 32-bit torus needs products exact to
-// well below the bootstrapping noise, which FP32 alone cannot give):
-//   * each integer key polynomial b is split into limbs
-//       hi = round(b / 2^24) in [-128, 128],  lo = b - hi * 2^24 in [-2^23, 2^23);
-//     both are transformed in FP64 on the device at key-load time and stored
-//     as FP32 frequency values;
-//   * per CMux the 6 digit polynomials (|d| <= 32) are transformed in FP32 and
-//     multiplied into four FP32 accumulators (hi/lo x 2 output polynomials);
-//   * the hi accumulators' inverse transforms are rounded to integers, which is
-//     exact: sum_r d_r * hi_r has rms magnitude ~2^16.7, so FP32 round-off
-//     (~2^-21.5 relative) leaves an error ~0.04, a 12-sigma margin below 1/2;
-//     then hi * 2^24 is taken modulo 2^32;
-//   * the lo accumulators' inverse transforms (rms ~2^32.7) are rounded to
-//     64-bit integers; their FP32 round-off (~2^11) is ~2^-6 of the per-CMux
-//     bootstrapping noise standard deviation (~2^17.8), i.e. it adds about
-//     0.03 % to the noise variance.
-// Kernel layout and key streaming are those of the FP64 kernel; the key ring
-// slots hold (hi, lo) float pairs in the same 16 KB per TRGSW row.
+// Batched lvl0 -> lvl1 programmable bootstrapping, split-precision FP32 path, with
+// the first step of every digit transform on the tensor cores (tc_stage1.cuh):
+// CUFHEDB_SPLIT32_TC.  The precision plan is the split path's (split_steps.cuh).
+// One warp per ciphertext, W per persistent CTA; the key streams through a ring
+// of shared-memory slots (ring.cuh) of one TRGSW row each, (hi, lo) float pairs
+// in 16 KB.
 #include "fft_f32.cuh"
 #include "pbs_common.cuh"
 #include "ring.cuh"
@@ -40,14 +24,13 @@ struct Pbs01SplitSmem {
     static constexpr int ACC_BYTES = 2 * N1 * 4;
     static constexpr int ABAR_BYTES = ((N0 * 2) + 127) / 128 * 128;
     static constexpr int PER_WARP = XP_BYTES + ACC_BYTES + ABAR_BYTES;
-    // tensor-core stage 1 only: the two FP16 limbs of B, one mbarrier per
-    // warp, the tensor-memory base address
+    // the two FP16 limbs of B, one mbarrier per warp, the tensor-memory base
+    // address
     static constexpr int TC_OFF = (WARP_OFF + W * PER_WARP + 1023) / 1024 * 1024;
     static constexpr int TC_B_BYTES = 2 * TC_B_HALVES * 2;
     static constexpr int TC_BAR_OFF = TC_OFF + TC_B_BYTES;
     static constexpr int TC_SLOT_OFF = TC_BAR_OFF + 8 * 16;
     static constexpr int TOTAL_TC = TC_SLOT_OFF + 16;
-    static constexpr int TOTAL = WARP_OFF + W * PER_WARP;
 };
 
 // Tensor-core stage 1 (tc_stage1.cuh), shared by the warps of a group of
@@ -151,11 +134,9 @@ static_assert(2 * TC_GROUP_COLS <= 512 && TC_D_COLS + 3 * 16 <= TC_GROUP_COLS,
               "two groups' columns within one SM's tensor memory");
 
 // W consumer warps, plus a producer warp when PRODUCER (ring.cuh has both
-// feeds; the launch picks per shape, see launch_pbs01_split).  TC: the first
-// step of every digit transform runs on the tensor cores (tc_stage1.cuh), the
-// rest as in the CUDA-core path.
-template <int W, int S, bool PRODUCER, bool TC>
-__global__ void __launch_bounds__((W + (PRODUCER ? 1 : 0)) * 32, 1) pbs01_split_kernel(Pbs01Args a)
+// feeds; the launch picks per shape, see launch_pbs01_split_tc)
+template <int W, int S, bool PRODUCER>
+__global__ void __launch_bounds__((W + (PRODUCER ? 1 : 0)) * 32, 1) pbs01_split_tc_kernel(Pbs01Args a)
 {
     // the folded tables (fft_f32.cuh): the twist and untwist ride on the
     // stage-1 twiddles, so the kernel reads 12.3 KB of tables instead of 24.4
@@ -174,29 +155,23 @@ __global__ void __launch_bounds__((W + (PRODUCER ? 1 : 0)) * 32, 1) pbs01_split_
     uint32_t *tc_slot = reinterpret_cast<uint32_t *>(smem + L::TC_SLOT_OFF);
     if (threadIdx.x == 0) {
         ring.init_by_thread0();
-        if constexpr (TC) {
-            for (int k = 0; k < 4; ++k) mbar_init(&tc_bars[k], 1);   // 2 groups x 2 buffers
-            fence_barrier_init();
-        }
+        for (int k = 0; k < 4; ++k) mbar_init(&tc_bars[k], 1);   // 2 groups x 2 buffers
+        fence_barrier_init();
     }
-    if constexpr (TC) {
-        if (warp == 0) tmem_alloc(tc_slot, tc_cols<W>());
-    }
+    if (warp == 0) tmem_alloc(tc_slot, tc_cols<W>());
     {
         const Fft512TablesF *all = reinterpret_cast<const Fft512TablesF *>(a.tables);
         const float4 *src = reinterpret_cast<const float4 *>(&all->fold);
         float4 *dst = reinterpret_cast<float4 *>(T);
         for (int i = threadIdx.x; i < (int)(sizeof(TT) / 16); i += blockDim.x) dst[i] = src[i];
-        if constexpr (TC) {
-            const float4 *bs = reinterpret_cast<const float4 *>(&all->tc_b[0][0]);
-            float4 *bd = reinterpret_cast<float4 *>(smem + L::TC_OFF);
-            for (int i = threadIdx.x; i < L::TC_B_BYTES / 16; i += blockDim.x) bd[i] = bs[i];
-            fence_proxy_async_smem();   // B is read by the tensor cores (async proxy)
-        }
+        const float4 *bs = reinterpret_cast<const float4 *>(&all->tc_b[0][0]);
+        float4 *bd = reinterpret_cast<float4 *>(smem + L::TC_OFF);
+        for (int i = threadIdx.x; i < L::TC_B_BYTES / 16; i += blockDim.x) bd[i] = bs[i];
+        fence_proxy_async_smem();   // B is read by the tensor cores (async proxy)
     }
-    if constexpr (TC) tc_fence_before();
+    tc_fence_before();
     __syncthreads();
-    if constexpr (TC) tc_fence_after();
+    tc_fence_after();
     if constexpr (PRODUCER) {
         if (warp == W) {
             ring.run_producer(lane, a.err);
@@ -228,7 +203,7 @@ __global__ void __launch_bounds__((W + (PRODUCER ? 1 : 0)) * 32, 1) pbs01_split_
             acc[N1 + j] = testvec_rot1(a.tv, j, bbar);
         }
         __syncwarp();
-        if constexpr (TC) {
+        {
             // polynomial 0's products of CMux 0; those of every later CMux are
             // issued between the previous CMux's two inverse transforms
             const uint32_t ab0 = valid ? abar_s[0] : 0u;
@@ -245,24 +220,16 @@ __global__ void __launch_bounds__((W + (PRODUCER ? 1 : 0)) * 32, 1) pbs01_split_
 #pragma unroll 1
             for (int r = 0; r < 2 * L1; ++r, ++c) {
                 float2 v[16];
-                if constexpr (TC) {
-                    if (r == 1) {
-                        // polynomial 1's products, under the transforms of
-                        // digits 1 and 2
-                        if (active) digit_words1(w, acc + N1, ab, lane);
-                        tc.put_issue(w, active, 1, warp, lane);
-                    }
-                    if (r % L1 == 0) tc.wait(r / L1, warp, a.err);
-                    tc.take(v, active, r, warp);
-                } else {
-                    if (active && r % L1 == 0) digit_words1(w, acc + (r / L1) * N1, ab, lane);
+                if (r == 1) {
+                    // polynomial 1's products, under the transforms of
+                    // digits 1 and 2
+                    if (active) digit_words1(w, acc + N1, ab, lane);
+                    tc.put_issue(w, active, 1, warp, lane);
                 }
+                if (r % L1 == 0) tc.wait(r / L1, warp, a.err);
+                tc.take(v, active, r, warp);
                 const float4 *bkc = reinterpret_cast<const float4 *>(ring.acquire(c, a.err));
                 if (active) {
-                    if constexpr (!TC) {
-                        digits_from_words_f(v, w, r % L1);
-                        fdft16<1>(v);
-                    }
                     ffft512_fwd_tw_rest(v, reinterpret_cast<float2 *>(xp), *T, lane);
                     if (r == 0) {
 #pragma unroll
@@ -286,24 +253,18 @@ __global__ void __launch_bounds__((W + (PRODUCER ? 1 : 0)) * 32, 1) pbs01_split_
                 }
                 ring.release(c, lane);
             }
-            if constexpr (TC) {
-                if (active) {
-                    add_inverse_split(acc, f0, xp, lane, *T);
-                    __syncwarp();
-                }
-                if (i + 1 < N0) {
-                    // the next CMux's polynomial 0 is final here: its products
-                    // run under this CMux's second inverse transform
-                    const uint32_t abn = valid ? abar_s[i + 1] : 0u;
-                    if (abn) digit_words1(w, acc, abn, lane);
-                    tc.put_issue(w, abn != 0, 0, warp, lane);
-                }
-                if (active) {
-                    add_inverse_split(acc + N1, f1, xp, lane, *T);
-                    __syncwarp();
-                }
-            } else if (active) {
+            if (active) {
                 add_inverse_split(acc, f0, xp, lane, *T);
+                __syncwarp();
+            }
+            if (i + 1 < N0) {
+                // the next CMux's polynomial 0 is final here: its products
+                // run under this CMux's second inverse transform
+                const uint32_t abn = valid ? abar_s[i + 1] : 0u;
+                if (abn) digit_words1(w, acc, abn, lane);
+                tc.put_issue(w, abn != 0, 0, warp, lane);
+            }
+            if (active) {
                 add_inverse_split(acc + N1, f1, xp, lane, *T);
                 __syncwarp();
             }
@@ -315,14 +276,12 @@ __global__ void __launch_bounds__((W + (PRODUCER ? 1 : 0)) * 32, 1) pbs01_split_
         }
         __syncwarp();
     }
-    if constexpr (TC) {
-        // every product of every warp was waited for; then the columns are freed
-        tc_fence_before();
-        asm volatile("bar.sync 1, %0;" ::"r"(W * 32) : "memory");
-        if (warp == 0) {
-            tc_fence_after();
-            tmem_dealloc(*tc_slot, tc_cols<W>());
-        }
+    // every product of every warp was waited for; then the columns are freed
+    tc_fence_before();
+    asm volatile("bar.sync 1, %0;" ::"r"(W * 32) : "memory");
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(*tc_slot, tc_cols<W>());
     }
     if constexpr (!PRODUCER) {
         __syncthreads();
@@ -338,65 +297,45 @@ constexpr int PBS01S_S = W == 8 ? 6 : 7;
 template <int W>
 using SplitLayout = Pbs01SplitSmem<W, PBS01S_S<W>, (int)sizeof(Fft512TablesFold)>;
 
-template <int W, bool TC>
-constexpr int split_smem_bytes()
-{
-    return TC ? SplitLayout<W>::TOTAL_TC : SplitLayout<W>::TOTAL;
-}
-
 // 7 and 4 ciphertexts per CTA run with a producer warp (8 or 5 warps), 8 per
 // CTA without one (8 warps): at most 2 warps per SM sub-partition (up to 255
 // registers); 4 per CTA leaves one consumer warp per sub-partition
 template <int W>
 constexpr bool PBS01S_PROD = W != 8;
 
-template <int W, bool TC>
-static cudaError_t launch_pbs01_split_t(const Pbs01Args &a, int grid, cudaStream_t st)
+template <int W>
+static cudaError_t launch_pbs01_split_tc_t(const Pbs01Args &a, int grid, cudaStream_t st)
 {
     constexpr bool PROD = PBS01S_PROD<W>;
-    static_assert(split_smem_bytes<W, TC>() <= 227 * 1024, "shared memory budget");
-    pbs01_split_kernel<W, PBS01S_S<W>, PROD, TC>
-        <<<grid, (W + (PROD ? 1 : 0)) * 32, split_smem_bytes<W, TC>(), st>>>(a);
+    static_assert(SplitLayout<W>::TOTAL_TC <= 227 * 1024, "shared memory budget");
+    pbs01_split_tc_kernel<W, PBS01S_S<W>, PROD>
+        <<<grid, (W + (PROD ? 1 : 0)) * 32, SplitLayout<W>::TOTAL_TC, st>>>(a);
     return cudaGetLastError();
-}
-
-template <bool TC>
-static cudaError_t launch_split_any(const Pbs01Args &a, int num_sms, int w, cudaStream_t st)
-{
-    if (a.B <= 0) return cudaSuccess;
-    const int groups = (a.B + w - 1) / w;
-    const int grid = groups < num_sms ? groups : num_sms;
-    if (w == 7) return launch_pbs01_split_t<7, TC>(a, grid, st);
-    if (w == 8) return launch_pbs01_split_t<8, TC>(a, grid, st);
-    if (w == 4) return launch_pbs01_split_t<4, TC>(a, grid, st);
-    return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_pbs01_split(const Pbs01Args &a, int num_sms, int w, cudaStream_t st)
-{
-    return launch_split_any<false>(a, num_sms, w, st);
 }
 
 cudaError_t launch_pbs01_split_tc(const Pbs01Args &a, int num_sms, int w, cudaStream_t st)
 {
-    return launch_split_any<true>(a, num_sms, w, st);
+    if (a.B <= 0) return cudaSuccess;
+    const int groups = (a.B + w - 1) / w;
+    const int grid = groups < num_sms ? groups : num_sms;
+    if (w == 7) return launch_pbs01_split_tc_t<7>(a, grid, st);
+    if (w == 8) return launch_pbs01_split_tc_t<8>(a, grid, st);
+    if (w == 4) return launch_pbs01_split_tc_t<4>(a, grid, st);
+    return cudaErrorInvalidValue;
 }
 
-template <int W, bool TC>
-static cudaError_t init_pbs01_split_t()
+template <int W>
+static cudaError_t init_pbs01_split_tc_t()
 {
-    return cudaFuncSetAttribute(pbs01_split_kernel<W, PBS01S_S<W>, PBS01S_PROD<W>, TC>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem_bytes<W, TC>());
+    return cudaFuncSetAttribute(pbs01_split_tc_kernel<W, PBS01S_S<W>, PBS01S_PROD<W>>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, SplitLayout<W>::TOTAL_TC);
 }
 
-cudaError_t init_pbs01_split()
+cudaError_t init_pbs01_split_tc()
 {
-    cudaError_t e = init_pbs01_split_t<7, false>();
-    if (e == cudaSuccess) e = init_pbs01_split_t<8, false>();
-    if (e == cudaSuccess) e = init_pbs01_split_t<4, false>();
-    if (e == cudaSuccess) e = init_pbs01_split_t<7, true>();
-    if (e == cudaSuccess) e = init_pbs01_split_t<8, true>();
-    if (e == cudaSuccess) e = init_pbs01_split_t<4, true>();
+    cudaError_t e = init_pbs01_split_tc_t<7>();
+    if (e == cudaSuccess) e = init_pbs01_split_tc_t<8>();
+    if (e == cudaSuccess) e = init_pbs01_split_tc_t<4>();
     return e;
 }
 

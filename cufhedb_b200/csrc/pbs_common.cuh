@@ -68,26 +68,26 @@ struct Pbs01Args {
     int *err;
 };
 
-// w: ciphertexts (warps) per CTA, one of PBS01_SHAPES
-cudaError_t launch_pbs01_f64(const Pbs01Args &a, int num_sms, int w, cudaStream_t st);
+// one ciphertext per CTA (pbs01_ct.cu)
+cudaError_t launch_pbs01_f64(const Pbs01Args &a, int num_sms, cudaStream_t st);
 // bk: split-precision key (float4 hi/lo chunk layout), tables: Fft512TablesF
-cudaError_t launch_pbs01_split(const Pbs01Args &a, int num_sms, int w, cudaStream_t st);
-// the same arithmetic, word for word, with 24 warps on one ciphertext per CTA
-// (pbs01_wide.cu)
-cudaError_t launch_pbs01_wide_f64(const Pbs01Args &a, int num_sms, cudaStream_t st);
-cudaError_t launch_pbs01_wide_split(const Pbs01Args &a, int num_sms, cudaStream_t st);
-// the same with the first step of every digit transform on the tensor cores
+cudaError_t launch_pbs01_split(const Pbs01Args &a, int num_sms, cudaStream_t st);
+cudaError_t init_pbs01_ct();
+// the split path with the first step of every digit transform on the tensor
+// cores (pbs01_split_tc.cu); w: ciphertexts (warps) per CTA, one of PBS01_SHAPES
 cudaError_t launch_pbs01_split_tc(const Pbs01Args &a, int num_sms, int w, cudaStream_t st);
+cudaError_t init_pbs01_split_tc();
 
-// Launch shapes of the persistent PBS kernels, as ciphertexts per CTA: lvl01
-// 7 (with a producer warp on the split path), 8 and 4 (one warp per SM
-// sub-partition: the shortest pass, for batches that leave SMs idle); lvl02
-// 3 (passes of 2, then of 1), 2 and 1.  Each CTA works through
-// ceil(ceil(B / w) / SMs) passes of w ciphertexts; the autotuner measures
-// one full pass of every shape, and a launch takes the shape with the least
-// passes x pass time.  Ties go to the earlier shape in the list, so with no
-// measurement (all pass times equal) the fewest passes win and a one-pass
-// batch runs 7 (lvl01) or 3 (lvl02) per CTA.
+// Launch shapes, the batch sizes per SM that the autotuner times a pass of:
+// lvl01 7, 8 and 4, lvl02 3, 2 and 1.  The tensor-core lvl01 kernel runs that
+// many ciphertexts per CTA (7 with a producer warp, 8, and 4: one warp per SM
+// sub-partition), lvl02 passes of 2 and of 1; the CUDA-core lvl01 kernel has one
+// ciphertext per CTA whatever the shape, and its times are estimates for the
+// scheduler and for the layout choice.  A batch of B takes ceil(ceil(B / w) /
+// SMs) passes; the shape with the least passes x pass time is taken.  Ties go
+// to the earlier shape in the list, so with no measurement (all pass times
+// equal) the fewest passes win and a one-pass batch counts as 7 (lvl01) or 3
+// (lvl02).
 constexpr int NSHAPES = 3;
 constexpr int PBS01_SHAPES[NSHAPES] = {7, 8, 4};
 constexpr int PBS02_SHAPES[NSHAPES] = {3, 2, 1};
@@ -145,18 +145,11 @@ inline int pbs02_choose_p(int B, int num_sms, const float pass_ms[NSHAPES])
 {
     return choose_shape(B, num_sms, PBS02_SHAPES, pass_ms);
 }
-// How one call's batch is run: up to two launches, each in a shape of the
-// table (w ciphertexts per CTA) or, w = 1 on lvl01, by the kernel that has all
-// of an SM on one ciphertext.  Every kernel of a path gives the same words, so
-// this is a choice of time only:
-//   * the whole batch in the shape the table picks;
-//   * the whole batch with one ciphertext per SM at a time;
-//   * full passes of one shape, and the rest, which would be a mostly empty
-//     pass, by whichever of the others is shortest for it.
-// `one_ratio` is the measured time of a pass of one ciphertext per SM over
-// that of the shape `one_of`; the estimate scales with the context's table, and
-// a table that was never measured is replaced by the times of a B200
-// (`b200_ms`).
+// How one lvl02 call's batch is run: up to two launches, each in a shape of the
+// table.  Every shape gives the same words, so this is a choice of time only: the
+// whole batch in the shape the table picks, or full passes of one shape and the
+// rest, which would be a mostly empty pass, in whichever is shortest for it.  A
+// table that was never measured is replaced by the times of a B200.
 struct BatchPart {
     int n;   // ciphertexts
     int w;   // per CTA
@@ -165,37 +158,19 @@ struct BatchPlan {
     int parts;
     BatchPart part[2];
 };
-struct ShapeTimes {
-    float b200_ms[NSHAPES];
-    int one_of;
-    float one_ratio;
-};
-// pass times (ms) on a B200 in the order of PBS01_SHAPES: 7, 8, 4 per CTA; one
-// ciphertext per SM 2.30 (split) and 3.18 (FP64) of the 4-per-CTA pass
-constexpr ShapeTimes PBS01_SPLIT_TIMES = {{9.40f, 10.31f, 7.50f}, 2, 0.307f};
-constexpr ShapeTimes PBS01_F64_TIMES = {{14.21f, 14.60f, 10.58f}, 2, 0.301f};
-
-// lvl02: 3, 2 and 1 ciphertexts per SM (the last is the table's own shape 1)
-constexpr ShapeTimes PBS02_TIMES = {{17.15f, 10.89f, 6.20f}, 2, 1.0f};
+// pass times (ms) on a B200: 3, 2 and 1 ciphertexts per SM
+constexpr float PBS02_B200_MS[NSHAPES] = {17.15f, 10.89f, 6.20f};
 
 inline BatchPlan plan_batch(int B, int num_sms, const int shapes[NSHAPES], const float pass_ms[NSHAPES],
-                            const ShapeTimes &times)
+                            const float b200_ms[NSHAPES])
 {
-    const float *ms = shape_table_measured(pass_ms) ? pass_ms : times.b200_ms;
-    const float one_ms = times.one_ratio * ms[times.one_of];
-    auto passes = [&](int n, int w) { return (float)(((n + w - 1) / w + num_sms - 1) / num_sms); };
-    // the best single launch for n ciphertexts: ties to the table's shapes
+    const float *ms = shape_table_measured(pass_ms) ? pass_ms : b200_ms;
+    // the best single launch for n ciphertexts
     auto single = [&](int n, int &w) {
-        const int s = choose_shape(n, num_sms, shapes, ms);
+        w = choose_shape(n, num_sms, shapes, ms);
         float cost = 0.0f;
         for (int i = 0; i < NSHAPES; ++i)
-            if (shapes[i] == s) cost = passes(n, s) * ms[i];
-        w = s;
-        const float one = passes(n, 1) * one_ms;
-        if (one < cost) {
-            w = 1;
-            cost = one;
-        }
+            if (shapes[i] == w) cost = (float)(((n + w - 1) / w + num_sms - 1) / num_sms) * ms[i];
         return cost;
     };
     BatchPlan best{1, {{B, 0}, {0, 0}}};
@@ -212,8 +187,5 @@ inline BatchPlan plan_batch(int B, int num_sms, const int shapes[NSHAPES], const
     }
     return best;
 }
-cudaError_t init_pbs01_f64();
-cudaError_t init_pbs01_split();
-cudaError_t init_pbs01_wide();
 
 }  // namespace cfdb

@@ -1,8 +1,22 @@
 // Steps of the split-precision lvl01 bootstrap that its kernels share
-// (pbs01_split.cu, pbs01_quad.cu): decomposition words and digits, the packed
-// products, the inverse transform into the accumulator.  Every kernel of the
-// path runs these same operations in the same order per value, so all of them
-// give the same words.
+// (pbs01_ct.cu, pbs01_split_tc.cu).
+//
+// Precision plan (the 32-bit torus needs products exact to well below the
+// bootstrapping noise, which FP32 alone cannot give):
+//   * each integer key polynomial b is split into limbs
+//       hi = round(b / 2^24) in [-128, 128],  lo = b - hi * 2^24 in [-2^23, 2^23);
+//     both are transformed in FP64 on the device at key-load time and stored
+//     as FP32 frequency values;
+//   * per CMux the 6 digit polynomials (|d| <= 32) are transformed in FP32 and
+//     multiplied into four FP32 accumulators (hi/lo x 2 output polynomials);
+//   * the hi accumulators' inverse transforms are rounded to integers, which is
+//     exact: sum_r d_r * hi_r has rms magnitude ~2^16.7, so FP32 round-off
+//     (~2^-21.5 relative) leaves an error ~0.04, a 12-sigma margin below 1/2;
+//     then hi * 2^24 is taken modulo 2^32;
+//   * the lo accumulators' inverse transforms (rms ~2^32.7) are rounded to
+//     64-bit integers; their FP32 round-off (~2^11) is ~2^-6 of the per-CMux
+//     bootstrapping noise standard deviation (~2^17.8), i.e. it adds about
+//     0.03 % to the noise variance.
 #pragma once
 #include "fft_f32.cuh"
 #include "pbs_common.cuh"
@@ -19,17 +33,6 @@ __device__ __forceinline__ void digit_words1(uint32_t w[32], const uint32_t *pol
         const int m = lane + 32 * m2;
         w[2 * m2] = ((rot_coef<N1>(poly, m, abar) - poly[m]) + DEC1_OFFSET + DEC1_ROUND) ^ DEC1_XOR;
         w[2 * m2 + 1] = ((rot_coef<N1>(poly, m + 512, abar) - poly[m + 512]) + DEC1_OFFSET + DEC1_ROUND) ^ DEC1_XOR;
-    }
-}
-
-// v[m2] = (dig_d(m) + i dig_d(m+512)) * w^{32 m2} from the cached words: the
-// per-register part of the twist (ffft512_fwd_tw applies the lane's part)
-__device__ __forceinline__ void digits_from_words_f(float2 v[16], const uint32_t w[32], int d)
-{
-#pragma unroll
-    for (int m2 = 0; m2 < 16; ++m2) {
-        const int d0 = digit_field1(w[2 * m2], d), d1 = digit_field1(w[2 * m2 + 1], d);
-        v[m2] = cw64(make_float2((float)d0, (float)d1), m2);
     }
 }
 

@@ -386,20 +386,20 @@ CUFHEDB_API int cufhedb_compare_host_multi(cufhedb_ctx *const *ctxs, int nctx, i
 CUFHEDB_API int cufhedb_selftest_wait_timeout(cufhedb_ctx *ctx, uint32_t polls);
 
 /* ---- launch-shape autotuner --------------------------------------------------- */
-/* The persistent PBS kernels come in three launch shapes each (ciphertexts
- * per CTA): lvl01 7, 8 and 4, lvl02 3, 2 and 1.  A launch of B ciphertexts
- * takes ceil(ceil(B / shape) / SMs) passes; every launch (PBS, gates,
- * operator chains) picks the shape with the least passes x measured pass
- * time, ties to the earlier shape; without measurements all pass times count
- * as equal.  The lvl01 paths (not CUFHEDB_SPLIT32_TC) may divide a batch:
- * a small batch, or what is left after a shape's full passes, runs on a
- * kernel with one ciphertext per SM or in another shape where that is
- * shorter; the results are the same words.  CUFHEDB_SPLIT32 launches also
- * pick the layout of the first transform step, on the CUDA cores or on the
- * tensor cores (the CUFHEDB_SPLIT32_TC kernel), by the same rule over both
- * tables once both are measured, ties to the CUDA cores.  No counterpart in the reference,
- * which runs one ciphertext per launch.  The tuning calls are synchronous;
- * call them outside stream capture. */
+/* Launch shapes are ciphertexts per SM in a pass: lvl01 7, 8 and 4, lvl02 3, 2
+ * and 1.  A batch of B takes ceil(ceil(B / shape) / SMs) passes; the shape with
+ * the least passes x measured pass time is taken, ties to the earlier shape;
+ * without measurements all pass times count as equal.  lvl02 and
+ * CUFHEDB_SPLIT32_TC launch in the shape (an lvl02 batch may be divided into
+ * full passes of one shape and a rest in another where that is shorter);
+ * CUFHEDB_FP64 and CUFHEDB_SPLIT32 on the CUDA cores run one ciphertext per
+ * block whatever the shape, and their times serve the queue scheduler and the
+ * next choice: CUFHEDB_SPLIT32 launches pick the layout of the first transform
+ * step, on the CUDA cores or on the tensor cores (the CUFHEDB_SPLIT32_TC
+ * kernel), by the same rule over both tables once both are measured, ties to
+ * the CUDA cores.  The results are the same words in every shape.  No
+ * counterpart in the reference, which runs one ciphertext per launch.  The
+ * tuning calls are synchronous; call them outside stream capture. */
 /* times one full pass of each lvl01 shape for `precision` (uniform random lvl0
  * inputs, the loaded key) and keeps them in the context; ms_w7 / ms_w8 (may be
  * NULL) receive the 7- and 8-per-CTA pass times */

@@ -1,4 +1,4 @@
-"""How a call's batch is divided over kernels and launch shapes (plan_batch in
+"""How an lvl02 call's batch is divided over launches (plan_batch in
 csrc/pbs_common.cuh), compiled for the host: every plan covers the batch
 exactly once, a two-part plan starts with whole passes of its shape, and no
 plan is estimated slower than any single launch."""
@@ -11,8 +11,8 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "cufhedb_b200", "csrc")
 SMS, BMAX = 148, 4000
-SHAPES = (7, 8, 4)
-TIMES = {"split": ((9.40, 10.31, 7.50), 0.307), "f64": ((14.21, 14.60, 10.58), 0.301)}
+SHAPES = (3, 2, 1)
+DEFAULT = (17.15, 10.89, 6.20)
 
 PROG = r"""
 #include "pbs_common.cuh"
@@ -20,11 +20,9 @@ PROG = r"""
 #include <cstdlib>
 int main(int argc, char **argv)
 {
-    const bool f64 = argv[1][0] == 'f';
-    const float ms[3] = {(float)atof(argv[2]), (float)atof(argv[3]), (float)atof(argv[4])};
+    const float ms[3] = {(float)atof(argv[1]), (float)atof(argv[2]), (float)atof(argv[3])};
     for (int B = 1; B <= %d; ++B) {
-        const cfdb::BatchPlan p =
-            cfdb::plan_batch(B, %d, cfdb::PBS01_SHAPES, ms, f64 ? cfdb::PBS01_F64_TIMES : cfdb::PBS01_SPLIT_TIMES);
+        const cfdb::BatchPlan p = cfdb::plan_batch(B, %d, cfdb::PBS02_SHAPES, ms, cfdb::PBS02_B200_MS);
         std::printf("%%d", p.parts);
         for (int k = 0; k < p.parts; ++k) std::printf(" %%d %%d", p.part[k].n, p.part[k].w);
         std::printf("\n");
@@ -46,22 +44,18 @@ def exe(tmp_path_factory):
     return str(d / "plan")
 
 
-@pytest.mark.parametrize("path", ["split", "f64"])
-@pytest.mark.parametrize("table", ["untuned", "tuned", "forced_7", "forced_4"])
-def test_plans_cover_the_batch_and_beat_single_launches(exe, path, table):
-    default, ratio = TIMES[path]
-    ms = {"untuned": (1.0, 1.0, 1.0), "tuned": tuple(1.07 * t for t in default), "forced_7": (0.001, 1000.0, 1000.0),
-          "forced_4": (1000.0, 1000.0, 0.001)}[table]
-    out = subprocess.run([exe, path, *map(repr, ms)], check=True, capture_output=True, text=True).stdout.split("\n")
-    t = dict(zip(SHAPES, default if table == "untuned" else ms))
-    t[1] = ratio * t[4]
+@pytest.mark.parametrize("ms", [(1.0, 1.0, 1.0), (18.0, 11.2, 6.5), (17.7, 13.8, 10.3), (0.001, 1000.0, 1000.0),
+                                (1000.0, 1000.0, 0.001)])
+def test_plans_cover_the_batch_and_beat_single_launches(exe, ms):
+    out = subprocess.run([exe, *map(repr, ms)], check=True, capture_output=True, text=True).stdout.split("\n")
+    t = dict(zip(SHAPES, DEFAULT if ms == (1.0, 1.0, 1.0) else ms))
     cost = lambda n, w: -(-(-(-n // w)) // SMS) * t[w]
     for B in range(1, BMAX + 1):
         f = [int(x) for x in out[B - 1].split()]
         parts = list(zip(f[1::2], f[2::2]))
         assert len(parts) == f[0] <= 2 and sum(n for n, _ in parts) == B and all(n > 0 for n, _ in parts)
-        if len(parts) == 2:
-            assert parts[0][1] in SHAPES and parts[0][0] % (parts[0][1] * SMS) == 0
         assert all(w in t for _, w in parts)
+        if len(parts) == 2:
+            assert parts[0][0] % (parts[0][1] * SMS) == 0
         planned = sum(cost(n, w) for n, w in parts)
         assert planned <= min(cost(B, w) for w in t) * (1 + 1e-5), (B, parts)

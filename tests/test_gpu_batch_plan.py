@@ -1,7 +1,7 @@
-"""GPU: the lvl01 kernel with one ciphertext per SM, and batches divided over
-two launches, against one launch of the one-warp-per-ciphertext kernel: equal
-words for every row.  The lvl02 kernel with one and two ciphertexts per CTA and
-its divided batches against one another."""
+"""GPU: a bootstrap's words do not depend on the batch it is in.  lvl01: every
+launch variant of the batch size (one, two to three, four and more ciphertexts
+per SM) gives a row the words it has in a large batch.  lvl02: every shape, and
+batches divided over two launches, give the same words."""
 from __future__ import annotations
 
 import pytest
@@ -10,28 +10,6 @@ from conftest import SEED
 
 pytestmark = pytest.mark.gpu
 N0, N1, N2 = 672, 1024, 2048
-
-
-@pytest.fixture(scope="module")
-def engines(tmp_path_factory):
-    """(engine whose table makes the 7-per-CTA shape the only short one, so
-    every batch is one launch of it; engine with the untuned table)"""
-    from cufhedb_b200 import GEN_BK01, Engine
-    one_warp, divided = Engine(0), Engine(0)
-    for e in (one_warp, divided):
-        e.keygen(SEED, GEN_BK01)
-    path = str(tmp_path_factory.mktemp("tbl") / "t.tbl")
-    one_warp.autotune_save(path)
-    lines = open(path).read().splitlines()
-    for i, ln in enumerate(lines):
-        if ln.startswith(("pbs01 fp64 ", "pbs01 split32 ")):
-            f = ln.split()
-            lines[i] = " ".join(f[:2] + [x for w in f[2::2] for x in (w, "0.001" if w == "7" else "1000.0")])
-    open(path, "w").write("\n".join(lines) + "\n")
-    assert one_warp.autotune_load(path)
-    yield one_warp, divided
-    one_warp.close()
-    divided.close()
 
 
 @pytest.fixture(scope="module")
@@ -92,20 +70,21 @@ def _inputs(B):
 
 @pytest.mark.parametrize("precision", ["split32", "fp64"])
 @pytest.mark.parametrize("tv", ["const", "staircase", "poly"])
-@pytest.mark.parametrize("rows", [1, 2, "sms", "sms+1", "8sms+3"])
-def test_words_equal_the_one_warp_kernel(engines, precision, tv, rows):
+def test_lvl01_words_do_not_depend_on_the_batch(precision, tv):
     import torch
-    from cufhedb_b200 import FP64, SPLIT32, testvec_const, testvec_poly, testvec_staircase
-    one_warp, divided = engines
+    from cufhedb_b200 import FP64, GEN_BK01, SPLIT32, Engine, testvec_const, testvec_poly, testvec_staircase
     prec = SPLIT32 if precision == "split32" else FP64
-    S = divided.num_sms
-    B = {"sms": S, "sms+1": S + 1, "8sms+3": 8 * S + 3}.get(rows, rows)
-    poly = torch.arange(N1, device="cuda", dtype=torch.int32) * 2097143
-    vec = {"const": testvec_const(1 << 29), "staircase": testvec_staircase(20), "poly": testvec_poly(poly)}[tv]
-    x = _inputs(B)
-    out = [torch.empty(B * (N1 + 1), dtype=torch.int32, device="cuda") for _ in range(2)]
-    one_warp.pbs_lvl01(x, out[0], vec, prec)
-    divided.pbs_lvl01(x, out[1], vec, prec)
-    one_warp.sync()
-    divided.sync()
-    assert torch.equal(out[0], out[1])
+    with Engine(0) as eng:
+        eng.keygen(SEED, GEN_BK01)
+        S = eng.num_sms
+        B = 4 * S + 5
+        poly = torch.arange(N1, device="cuda", dtype=torch.int32) * 2097143
+        vec = {"const": testvec_const(1 << 29), "staircase": testvec_staircase(20), "poly": testvec_poly(poly)}[tv]
+        x = _inputs(B)
+        want = torch.empty(B * (N1 + 1), dtype=torch.int32, device="cuda")
+        eng.pbs_lvl01(x, want, vec, prec)
+        for n in (1, 2, S, S + 1, 2 * S + 1, 3 * S + 1):
+            got = torch.empty(n * (N1 + 1), dtype=torch.int32, device="cuda")
+            eng.pbs_lvl01(x[: n * (N0 + 1)].contiguous(), got, vec, prec)
+            eng.sync()
+            assert torch.equal(got, want[: n * (N1 + 1)]), n
