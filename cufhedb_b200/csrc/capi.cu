@@ -1222,7 +1222,7 @@ int cufhedb_extprod_lvl1(cufhedb_ctx *ctx, const uint32_t *trlwe, const void *tr
     a.B = B;
     a.shared = shared ? 1 : 0;
     a.tables = precision == CUFHEDB_FP64 ? (const void *)ctx->tab512 : (const void *)ctx->tab512f;
-    a.err = ctx->err;
+    a.num_sms = ctx->num_sms;
     CK(launch_extprod1(a, precision == CUFHEDB_FP64 ? 0 : 1, (cudaStream_t)stream));
     return CUFHEDB_OK;
 }
@@ -1390,7 +1390,7 @@ int cufhedb_extprod_lvl1_host(cufhedb_ctx *ctx, const uint32_t *trlwe, const dou
         a.B = B;
         a.shared = shared ? 1 : 0;
         a.tables = ctx->tab512;
-        a.err = ctx->err;
+        a.num_sms = ctx->num_sms;
         e = launch_extprod1(a, 0, st);
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, dout, tb, cudaMemcpyDeviceToHost, st);

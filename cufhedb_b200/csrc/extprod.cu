@@ -4,241 +4,117 @@
 //
 // Restates trgswfftExternalProduct<lvl1param> (thirdparty/TFHEpp/src/
 // trgsw.cpp:77-103): res_o = sum_{k,d} IFFT(dec_d(trlwe_k)) * trgsw[k l + d][o],
-// transformed back per output polynomial.  One warp per product; the TRGSW
-// rows (one per TRGSW or one shared by the batch) are stored in the per-lane
-// chunk layout the PBS kernels use, and each TRGSW byte is read once.  The
-// FP64 kernel reads them straight from global memory.  In the split kernel
-// every warp copies its product's TRGSW row by row into its own 16 KB of
-// shared memory (a bulk copy completing on the warp's mbarrier), the copy of
-// row r + 1 issued as soon as the products of row r are read out, so it runs
-// under the transform of digit polynomial r + 1; lane 0 also asks L2 for the
-// rows two ahead (a bulk prefetch), so each copy finds its row there.  Waits
-// are bounded: a warp that gives up records DEV_TIMEOUT_ROW, issues no
-// further copy and, before it exits, waits (bounded again) for the one it
-// gave up on.
-
+// transformed back per output polynomial.
+//
+// A block of six or eight warps takes one product at a time through the steps of
+// a CMux (block_fft.cuh, pbs01_ct.cu), several blocks per SM, each looping over
+// products.  The next product's TRLWE and TRGSW are asked into L2 when one's
+// products are done (a whole product ahead, the blocks' 2 x 57 MB evicted one
+// another: 716 MB from DRAM instead of 450).  The TRGSW rows (one per TRGSW or one shared by the batch) are stored
+// in the per-lane chunk layout the bootstrapping keys use, and each TRGSW byte is
+// read once.  4,096 products: split 92 us (5.1 TB/s; DRAM floor 72), FP64 99 us,
+// shared 73 and 89; one warp per product, its row staged by bulk copies, took 131,
+// 144, 99 and 116.  One product: 20 us, was 31.
+#include "block_fft.cuh"
 #include "extprod.cuh"
-#include "fft_f32.cuh"
 
 namespace cfdb {
 
 namespace {
 
-// 16 KB per TRGSW row (1,024 complex FP64, or 1,024 (hi, lo) FP32 pairs)
-constexpr uint32_t TRGSW_ROW_BYTES = 16384;
-constexpr int EP_WARPS = 4;   // products (warps) per CTA
+// 96 KB per TRGSW: 6 rows of 1,024 complex FP64, or 1,024 (hi, lo) FP32 pairs
+constexpr uint32_t TRGSW_BYTES = 2 * L1 * 16384;
 
-// dynamic shared memory of a CTA: per warp a staged TRGSW row and its
-// transpose scratch (XPB bytes), then one mbarrier per warp
-template <int XPB>
-constexpr int ep_smem_bytes()
-{
-    return EP_WARPS * (int)TRGSW_ROW_BYTES + EP_WARPS * XPB + EP_WARPS * 8;
-}
-
-// one warp's TRGSW row staged in shared memory (see the file comment)
-struct RowStage {
-    unsigned char *buf;   // TRGSW_ROW_BYTES, 128-byte aligned
-    uint64_t *bar;
-    uint32_t phase;
-    bool ok;              // warp-uniform: no wait has given up
-
-    __device__ __forceinline__ void init(int lane)
-    {
-        if (lane == 0) {
-            mbar_init(bar, 1);
-            fence_barrier_init();
-        }
-        __syncwarp();
-    }
-    // after every lane's last read of the buffer (callers __syncwarp first)
-    __device__ __forceinline__ void issue(const unsigned char *row, int lane)
-    {
-        if (lane == 0 && ok) {
-            fence_proxy_async_smem();
-            mbar_arrive_expect_tx(bar, TRGSW_ROW_BYTES);
-            bulk_g2s(buf, row, TRGSW_ROW_BYTES, bar);
-        }
-    }
-    __device__ __forceinline__ void wait(int *err, int lane)
-    {
-        if (!ok) return;
-        const bool done = __all_sync(0xffffffffu, mbar_wait(bar, phase));
-        if (done) {
-            phase ^= 1;
-        } else {
-            ok = false;
-            if (lane == 0) report_error(err, DEV_TIMEOUT_ROW);
-        }
-    }
-    // a copy given up on may still be in flight: wait for it (bounded)
-    __device__ __forceinline__ void drain(int *err, int lane)
-    {
-        if (ok) return;
-        const bool done = __all_sync(0xffffffffu, mbar_wait(bar, phase));
-        if (!done && lane == 0) report_error(err, DEV_TIMEOUT_DRAIN);
-    }
+template <class P>
+struct EpSmem {
+    static constexpr int TAB_OFF = 64;
+    static constexpr int BUF_OFF = TAB_OFF + ((int)sizeof(typename P::Tab) + 63) / 64 * 64;
+    static constexpr int TOTAL = BUF_OFF + 2 * L1 * P::BUF * (int)sizeof(typename P::V);
 };
 
-// rows r and r + 1 of this warp's own TRGSW into L2 (nothing to do when the
-// batch shares one TRGSW: it stays in L2 anyway)
-__device__ __forceinline__ void prefetch_rows(const void *g, int r, int n, const ExtProdArgs &a, int lane)
+template <class P, int NW, int OCC>
+__global__ void __launch_bounds__(32 * NW, OCC) extprod1_kernel(ExtProdArgs a)
 {
-    if (a.shared || lane != 0) return;
-    for (int k = r; k < r + n && k < 2 * L1; ++k)
-        bulk_prefetch_l2(reinterpret_cast<const unsigned char *>(g) + (size_t)k * TRGSW_ROW_BYTES, TRGSW_ROW_BYTES);
-}
-
-__device__ __forceinline__ void digits_f64(double2 v[16], const uint32_t *poly, int d, int lane, const Fft512Tables &T)
-{
-    const int sh = 32 - BGBIT1 * (d + 1);
-#pragma unroll
-    for (int m2 = 0; m2 < 16; ++m2) {
-        const int m = lane + 32 * m2;
-        int d0 = (int)(((poly[m] + DEC1_OFFSET + DEC1_ROUND) >> sh) & 63u) - 32;
-        int d1 = (int)(((poly[m + 512] + DEC1_OFFSET + DEC1_ROUND) >> sh) & 63u) - 32;
-        v[m2] = cmul(make_double2((double)d0, (double)d1), T.twist[m2 * 32 + lane]);
-    }
-}
-
-__device__ __forceinline__ void digits_f32(float2 v[16], const uint32_t *poly, int d, int lane,
-                                           const Fft512TablesPlain &T)
-{
-    const int sh = 32 - BGBIT1 * (d + 1);
-#pragma unroll
-    for (int m2 = 0; m2 < 16; ++m2) {
-        const int m = lane + 32 * m2;
-        int d0 = (int)(((poly[m] + DEC1_OFFSET + DEC1_ROUND) >> sh) & 63u) - 32;
-        int d1 = (int)(((poly[m + 512] + DEC1_OFFSET + DEC1_ROUND) >> sh) & 63u) - 32;
-        v[m2] = fcmul(make_float2((float)d0, (float)d1), T.twist[m2 * 32 + lane]);
-    }
-}
-
-// The FP64 kernel reads its TRGSW rows straight from global memory: staged
-// through shared memory like the split kernel it measured slower (4,096
-// products 0.145 -> 0.190 ms).
-__global__ void __launch_bounds__(EP_WARPS * 32) extprod1_f64_kernel(ExtProdArgs a)
-{
-    __shared__ double2 xp_s[EP_WARPS][FFT512_XP];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int p = blockIdx.x * EP_WARPS + w;
-    if (p >= a.B) return;
-    double2 *xp = xp_s[w];
-    const Fft512Tables &T = *reinterpret_cast<const Fft512Tables *>(a.tables);
-    const uint32_t *in = a.trlwe + (size_t)p * 2 * N1;
-    if (lane == 0) bulk_prefetch_l2_if_aligned(in, 2 * N1 * sizeof(uint32_t));   // the TRLWE, read per digit
-    const double2 *g = reinterpret_cast<const double2 *>(a.trgsw) + (a.shared ? 0 : (size_t)p * 6 * 1024);
-    double2 f0[16], f1[16];
-#pragma unroll 1
-    for (int r = 0; r < 2 * L1; ++r) {
-        double2 v[16];
-        digits_f64(v, in + (r / L1) * N1, r % L1, lane, T);
-        fft512_fwd(v, xp, T, lane);
-        const double2 *gc = g + (size_t)r * 1024;
-        if (r == 0) {
-#pragma unroll
-            for (int s = 0; s < 16; ++s) {
-                f0[s] = cmul(v[s], gc[(2 * s) * 32 + lane]);
-                f1[s] = cmul(v[s], gc[(2 * s + 1) * 32 + lane]);
-            }
-        } else {
-#pragma unroll
-            for (int s = 0; s < 16; ++s) {
-                cfma(f0[s], v[s], gc[(2 * s) * 32 + lane]);
-                cfma(f1[s], v[s], gc[(2 * s + 1) * 32 + lane]);
-            }
-        }
-    }
-    uint32_t *o = a.out + (size_t)p * 2 * N1;
-    fft512_inv(f0, xp, T, lane);
-#pragma unroll
-    for (int m2 = 0; m2 < 16; ++m2) {
-        const int m = lane + 32 * m2;
-        const double2 y = cmulc(f0[m2], T.twist[m2 * 32 + lane]);
-        o[m] = f64_to_torus32(y.x * (1.0 / 512.0));
-        o[m + 512] = f64_to_torus32(y.y * (1.0 / 512.0));
-    }
-    fft512_inv(f1, xp, T, lane);
-#pragma unroll
-    for (int m2 = 0; m2 < 16; ++m2) {
-        const int m = lane + 32 * m2;
-        const double2 y = cmulc(f1[m2], T.twist[m2 * 32 + lane]);
-        o[N1 + m] = f64_to_torus32(y.x * (1.0 / 512.0));
-        o[N1 + m + 512] = f64_to_torus32(y.y * (1.0 / 512.0));
-    }
-}
-
-// o = the torus32 polynomial of the paired (hi, lo) frequency accumulator f:
-// round(hi) * 2^24 + round(lo) (mod 2^32)
-__device__ __forceinline__ void store_split(uint32_t *o, CP f[16], unsigned long long *xp, int lane,
-                                            const Fft512TablesPlain &T)
-{
-    pfft512_inv<false>(f, xp, T, lane);
-#pragma unroll
-    for (int m2 = 0; m2 < 16; ++m2) {
-        const int m = lane + 32 * m2;
-        const CP y = pmul_t(f[m2], T.untwistp[m2 * 32 + lane]);
-        const float2 re = unpk2(y.re), im = unpk2(y.im);
-        o[m] = ((uint32_t)__float2int_rn(re.x) << 24) + (uint32_t)__float2ll_rn(re.y);
-        o[m + 512] = ((uint32_t)__float2int_rn(im.x) << 24) + (uint32_t)__float2ll_rn(im.y);
-    }
-}
-
-// both limbs of one output: f (+)= v * k, k = (hi.re, lo.re, hi.im, lo.im)
-__device__ __forceinline__ void pmac_limbs(CP &f, float2 v, float4 k, bool first)
-{
-    const unsigned long long vr = pk2(v.x, v.x), vi = pk2(v.y, v.y), nvi = pk2(-v.y, -v.y);
-    const unsigned long long kr = pk2(k.x, k.y), ki = pk2(k.z, k.w);
-    if (first) {
-        f.re = f2(nvi, ki, m2(vr, kr));
-        f.im = f2(vi, kr, m2(vr, ki));
-    } else {
-        f.re = f2(nvi, ki, f2(vr, kr, f.re));
-        f.im = f2(vi, kr, f2(vr, ki, f.im));
-    }
-}
-
-constexpr int XPB_SPLIT = FFT512_XP * (int)sizeof(unsigned long long);
-
-__global__ void __launch_bounds__(EP_WARPS * 32) extprod1_split_kernel(ExtProdArgs a)
-{
+    using L = EpSmem<P>;
+    using V = typename P::V;
+    constexpr int BUF = P::BUF;
+    static_assert(NW >= 2 * L1, "one warp per row");
     extern __shared__ __align__(128) unsigned char smem[];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int p = blockIdx.x * EP_WARPS + w;
-    if (p >= a.B) return;
-    unsigned long long *xp =
-        reinterpret_cast<unsigned long long *>(smem + EP_WARPS * TRGSW_ROW_BYTES + w * XPB_SPLIT);
-    RowStage rs{smem + w * TRGSW_ROW_BYTES,
-                reinterpret_cast<uint64_t *>(smem + EP_WARPS * (TRGSW_ROW_BYTES + XPB_SPLIT)) + w, 0u, true};
-    rs.init(lane);
-    const Fft512TablesPlain &T = reinterpret_cast<const Fft512TablesF *>(a.tables)->plain;
-    const uint32_t *in = a.trlwe + (size_t)p * 2 * N1;
-    if (lane == 0) bulk_prefetch_l2_if_aligned(in, 2 * N1 * sizeof(uint32_t));   // the TRLWE, read per digit
-    const unsigned char *g = reinterpret_cast<const unsigned char *>(a.trgsw) +
-                             (a.shared ? 0 : (size_t)p * 2 * L1 * TRGSW_ROW_BYTES);
-    prefetch_rows(g, 1, 2, a, lane);
-    rs.issue(g, lane);
-    CP f0[16], f1[16];
-#pragma unroll 1
-    for (int r = 0; r < 2 * L1; ++r) {
-        float2 v[16];
-        prefetch_rows(g, r + 3, 1, a, lane);
-        digits_f32(v, in + (r / L1) * N1, r % L1, lane, T);
-        ffft512_fwd(v, reinterpret_cast<float2 *>(xp), T, lane);
-        rs.wait(a.err, lane);
-        const float4 *gc = reinterpret_cast<const float4 *>(rs.buf);
+    uint32_t *slot = reinterpret_cast<uint32_t *>(smem);
+    typename P::Tab *T = reinterpret_cast<typename P::Tab *>(smem + L::TAB_OFF);
+    V *buf = reinterpret_cast<V *>(smem + L::BUF_OFF);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // asks the TRLWE and the TRGSW of product p into L2
+    auto prefetch = [&](int p) {
+        if (tid != 0 || p >= a.B) return;
+        bulk_prefetch_l2_if_aligned(a.trlwe + (size_t)p * 2 * N1, 2 * N1 * sizeof(uint32_t));
+        if (!a.shared) bulk_prefetch_l2(reinterpret_cast<const unsigned char *>(a.trgsw) + (size_t)p * TRGSW_BYTES, TRGSW_BYTES);
+    };
+    prefetch(blockIdx.x);
+    const float4 *tab = P::tables(a.tables);
+    if (tid < (int)(sizeof(typename P::Tab) / 16)) reinterpret_cast<float4 *>(T)[tid] = tab[P::TAB_WORD4 + tid];
+    if (warp == 0) tmem_alloc(slot, P::COLS);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tm = *slot + ((32u * (warp & 3)) << 16);   // this sub-partition's lanes
+    if (warp < 4) P::stage_tables(tm, *reinterpret_cast<const typename P::Full *>(tab), lane);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+
+    for (int p = blockIdx.x; p < a.B; p += gridDim.x) {
+        const uint32_t *in = a.trlwe + (size_t)p * 2 * N1;
+        const float4 *g = reinterpret_cast<const float4 *>(a.trgsw) + (a.shared ? 0 : (size_t)p * (TRGSW_BYTES / 16)) + lane;
 #pragma unroll
-        for (int s = 0; s < 16; ++s) {
-            pmac_limbs(f0[s], v[s], gc[(2 * s) * 32 + lane], r == 0);
-            pmac_limbs(f1[s], v[s], gc[(2 * s + 1) * 32 + lane], r == 0);
+        for (int it = 0; it < (32 + NW - 1) / NW; ++it) {
+            const int row = warp + NW * it;   // (polynomial, m2), m = lane + 32 m2
+            if (row < 32) {
+                const int pol = row >> 4, m = lane + 32 * (row & 15);
+                put_digits<P>(buf + L1 * pol * BUF, m, in[pol * N1 + m], in[pol * N1 + m + 512]);
+            }
         }
-        __syncwarp();
-        if (r + 1 < 2 * L1) rs.issue(g + (size_t)(r + 1) * TRGSW_ROW_BYTES, lane);
+        __syncthreads();
+        if (warp < 2 * L1) {
+            V v[16];
+            V *xp = buf + warp * BUF;
+            P::forward(v, xp, lane, tm);
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) xp[32 * j + lane] = v[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int it = 0; it < (8 + NW - 1) / NW; ++it)
+            if (warp + NW * it < 8) products<P>(buf, g, *T, warp + NW * it, lane);
+        __syncthreads();
+        prefetch(p + gridDim.x);
+        uint32_t *o = a.out + (size_t)p * 2 * N1;
+        if (warp < P::INV)
+            P::inverse(buf + warp * BUF, buf + (warp ^ 1) * BUF, warp, lane, tm, [&](int m, uint32_t x) { o[m] = x; });
+        __syncthreads();
     }
-    rs.drain(a.err, lane);
-    uint32_t *o = a.out + (size_t)p * 2 * N1;
-    store_split(o, f0, xp, lane, T);
-    store_split(o + N1, f1, xp, lane, T);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(*slot, P::COLS);
+    }
+}
+
+template <class P, int NW, int OCC>
+cudaError_t launch_ep_t(const ExtProdArgs &a, cudaStream_t st)
+{
+    const int blocks = OCC * a.num_sms;
+    extprod1_kernel<P, NW, OCC><<<a.B < blocks ? a.B : blocks, 32 * NW, EpSmem<P>::TOTAL, st>>>(a);
+    return cudaGetLastError();
+}
+
+template <class P, int NW, int OCC>
+cudaError_t init_ep_t()
+{
+    return cudaFuncSetAttribute(extprod1_kernel<P, NW, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                EpSmem<P>::TOTAL);
 }
 
 }  // namespace
@@ -246,18 +122,22 @@ __global__ void __launch_bounds__(EP_WARPS * 32) extprod1_split_kernel(ExtProdAr
 cudaError_t launch_extprod1(const ExtProdArgs &a, int precision, cudaStream_t st)
 {
     if (a.B <= 0) return cudaSuccess;
-    const unsigned grid = (unsigned)((a.B + EP_WARPS - 1) / EP_WARPS);
+    // warps per block and blocks per SM as in pbs01_ct.cu, except that more than
+    // three split blocks per SM gain nothing where DRAM is the bound (us, 2 / 3 / 4
+    // per SM: 700 products 27.6 / 28.7 / 36.1; 4,096: 91.4 / 91.8 / 94.8, with a
+    // shared TRGSW 80.3 / 72.8 / 71.3)
     if (precision == 0)
-        extprod1_f64_kernel<<<grid, EP_WARPS * 32, 0, st>>>(a);
-    else
-        extprod1_split_kernel<<<grid, EP_WARPS * 32, ep_smem_bytes<XPB_SPLIT>(), st>>>(a);
-    return cudaGetLastError();
+        return a.B <= a.num_sms ? launch_ep_t<F64Path, 8, 2>(a, st) : launch_ep_t<F64Path, 6, 2>(a, st);
+    return a.B <= 2 * a.num_sms ? launch_ep_t<PlainPath, 8, 2>(a, st) : launch_ep_t<PlainPath, 8, 3>(a, st);
 }
 
 cudaError_t init_extprod1()
 {
-    return cudaFuncSetAttribute(extprod1_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                ep_smem_bytes<XPB_SPLIT>());
+    cudaError_t e = init_ep_t<PlainPath, 8, 2>();
+    if (e == cudaSuccess) e = init_ep_t<PlainPath, 8, 3>();
+    if (e == cudaSuccess) e = init_ep_t<F64Path, 8, 2>();
+    if (e == cudaSuccess) e = init_ep_t<F64Path, 6, 2>();
+    return e;
 }
 
 }  // namespace cfdb

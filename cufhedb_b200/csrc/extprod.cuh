@@ -11,7 +11,7 @@ struct ExtProdArgs {
     int B;
     int shared;              // 1: one TRGSW for the whole batch
     const void *tables;      // Fft512Tables (FP64 path) or Fft512TablesF (split path)
-    int *err;                // device error word (bounded waits that gave up)
+    int num_sms;
 };
 
 // precision 0: FP64, 1: split-precision FP32

@@ -88,3 +88,35 @@ def test_lvl01_words_do_not_depend_on_the_batch(precision, tv):
             eng.pbs_lvl01(x[: n * (N0 + 1)].contiguous(), got, vec, prec)
             eng.sync()
             assert torch.equal(got, want[: n * (N1 + 1)]), n
+
+
+@pytest.mark.parametrize("precision", ["split32", "fp64"])
+def test_lvl1_products_do_not_depend_on_the_batch(precision):
+    """external products: every launch variant of the batch size, a block's first
+    and later products, in place, and one shared TRGSW"""
+    import torch
+    from cufhedb_b200 import FP64, SPLIT32, Engine
+    prec = SPLIT32 if precision == "split32" else FP64
+    with Engine(0) as eng:
+        S = eng.num_sms
+        B = 4 * S + 5
+        g = torch.Generator(device="cuda").manual_seed(7)
+        words = lambda n: torch.randint(-2 ** 31, 2 ** 31, (n,), generator=g, device="cuda", dtype=torch.int32)
+        x, raw = words(B * 2 * N1), words(B * 6 * 2 * N1)
+        x[: 2 * N1] = -2 ** 31                       # extreme digits against extreme words
+        raw[: 12 * N1] = 2 ** 31 - 1
+        prep = torch.empty(B * 12288, dtype=torch.float64, device="cuda")
+        eng.trgsw_prepare_lvl1(raw, prep, prec)
+        want = torch.empty_like(x)
+        eng.extprod_lvl1(x, prep, want, precision=prec)
+        for n in (1, S, S + 1, 2 * S + 1):
+            got = x[: n * 2 * N1].clone()
+            eng.extprod_lvl1(got, prep[: n * 12288].contiguous(), got, precision=prec)
+            eng.sync()
+            assert torch.equal(got, want[: n * 2 * N1]), n
+        one = prep[:12288].contiguous()
+        got, rep = torch.empty_like(x), torch.empty_like(x)
+        eng.extprod_lvl1(x, one, got, shared=True, precision=prec)
+        eng.extprod_lvl1(x, one.repeat(B), rep, precision=prec)
+        eng.sync()
+        assert torch.equal(got, rep)
