@@ -24,13 +24,14 @@
 // (half of them the two transposes of each transform), 8,000 FP64-pipe cycles
 // and 8,000 issue slots per scheduler; at C = 2 the wavefronts run at 65 % of
 // their rate and FP64 at 49 %, the rest is the barriers and the latency between
-// the stages.  Pass times on a B200 (148 SMs): C = 1 6.20 ms, C = 2 10.89 ms,
+// the stages.  Pass times on a B200 (148 SMs): C = 1 5.72 ms, C = 2 10.89 ms,
 // where one team per ciphertext with both accumulators in its registers took
 // 10.26, 13.80 and, with three ciphertexts, 17.65 ms (the shape-3 launch here,
-// passes of two and of one: 17.1 ms).  On the way: all teams of both
+// passes of two and of one: 16.6 ms).  On the way: all teams of both
 // ciphertexts in lock step 12.28 ms; key chunks released by 16 warps with an
 // atomic each 8.49 ms at C = 1, by a producer warp (which costs the others
-// their registers) 7.06 ms; one release per team and round 6.20 ms.
+// their registers) 7.06 ms; one release per team and round 6.20 ms; each thread's
+// values loaded into its registers, ahead of the barrier, 5.72 ms.
 #include "lvl2_steps.cuh"
 #include "ring.cuh"
 #include "tc_stage1.cuh"
@@ -52,8 +53,10 @@ struct TeamShape {
     static constexpr int SL = 8 / TPC;
     static constexpr int CHUNK = 16384;                 // one (row, output): 1024 complex
     static constexpr int CHUNKS = 2 * TPC;              // per round
-    static constexpr int STAGED = C == 1 ? 7 : 4;       // of them in shared memory, the rest from global memory
-    static constexpr uint32_t BYTES = STAGED * CHUNK;
+    // two ciphertexts share the round's key in shared memory; one reads it into
+    // registers
+    static constexpr bool STAGED = C == 2;
+    static constexpr uint32_t BYTES = STAGED ? CHUNKS * CHUNK : 0;
     static constexpr int KEY_OFF = 128;
     static constexpr int TAB_OFF = KEY_OFF + (int)BYTES;
     static constexpr int XP_OFF = TAB_OFF + ((int)sizeof(Fft1024Tables) + 127) / 128 * 128;
@@ -134,6 +137,16 @@ __device__ __forceinline__ double2 get_c(const uint32_t *x)
     return make_double2(__hiloint2double((int)x[1], (int)x[0]), __hiloint2double((int)x[3], (int)x[2]));
 }
 
+// a read-only load issued where it stands
+__device__ __forceinline__ float4 ldg_here(const float4 *p)
+{
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p));
+    return v;
+}
+
 // the teams of a ciphertext meet; tensor-memory stores before it (waited for)
 // are visible to loads after it
 template <int C>
@@ -159,7 +172,7 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
     const int warp = threadIdx.x >> 5;
     const int team = threadIdx.x / T2, t = threadIdx.x % T2, bar = 1 + team;
     const int q = team / TPC, h = team % TPC;   // the ciphertext, and the team's place in it
-    if (threadIdx.x == 0) key.init();
+    if (S::STAGED && threadIdx.x == 0) key.init();
     if (warp == 0) tmem_alloc(slot, 512);
     {
         const double2 *src = reinterpret_cast<const double2 *>(a.tables);
@@ -169,7 +182,7 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (threadIdx.x == 0) key.issue(0);
+    if (S::STAGED && threadIdx.x == 0) key.issue(0);
     const uint32_t tm = *slot + ((32u * (warp & 3)) << 16);
 
     double2 *xp = reinterpret_cast<double2 *>(smem + S::XP_OFF + team * S::XP_BYTES);
@@ -193,7 +206,7 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
             const uint32_t ab = valid ? (an + (1u << 19)) >> 20 : 0u;
             an = in[i + 1];
             if (ab == 0) {
-                for (int k = 0; k < ROUNDS; ++k, ++n) {
+                for (int k = 0; S::STAGED && k < ROUNDS; ++k, ++n) {
                     key.acquire(n, a.err);
                     if (t == 0) key.release(n);
                 }
@@ -238,24 +251,28 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
                     // every thread of the team is past its products of the
                     // round before when it reaches the transform's first barrier
                     fft8x_fwd<double2, T2>(v, xp, *T, t, bar, [&] {
-                        if (k > 0 && t == 0) key.release(n - 1);
+                        if (S::STAGED && k > 0 && t == 0) key.release(n - 1);
                     });
 #pragma unroll
                     for (int s = 0; s < 8; ++s) put_c(x + 4 * s, v[s]);
                     tmem_st32_nowait(tm + TT_SPEC + 128 * (k & 1) + 32 * team, x);
                     tmem_wait_st();
                 }
-                ct_sync<C>(q);
                 // chunk e of the round: row TPC k + e / 2, output e % 2; this
-                // thread's values at [slot][t]
-                const float4 *kg = reinterpret_cast<const float4 *>(a.bk) +
-                                   ((size_t)(i * ROUNDS + k) * S::CHUNKS) * 1024 + SL * h * T2 + t;
-                float4 far[S::CHUNKS - S::STAGED + 1][SL];
+                // thread's values at [slot][t].  Read into registers they are
+                // asked for before the barrier, so the memory's latency runs
+                // under the wait for the slowest team.
+                float4 kr[S::STAGED ? 1 : S::CHUNKS][SL];
+                if constexpr (!S::STAGED) {
+                    const float4 *kg = reinterpret_cast<const float4 *>(a.bk) +
+                                       ((size_t)(i * ROUNDS + k) * S::CHUNKS) * 1024 + SL * h * T2 + t;
 #pragma unroll
-                for (int e = S::STAGED; e < S::CHUNKS; ++e)
+                    for (int e = 0; e < S::CHUNKS; ++e)
 #pragma unroll
-                    for (int s = 0; s < SL; ++s) far[e - S::STAGED][s] = __ldg(kg + e * 1024 + s * T2);
-                key.acquire(n, a.err);
+                        for (int s = 0; s < SL; ++s) kr[e][s] = ldg_here(kg + e * 1024 + s * T2);
+                }
+                ct_sync<C>(q);
+                if constexpr (S::STAGED) key.acquire(n, a.err);
                 const double2 *ks = reinterpret_cast<const double2 *>(smem + S::KEY_OFF) + SL * h * T2 + t;
 #pragma unroll
                 for (int rr = 0; rr < TPC; ++rr) {
@@ -270,8 +287,9 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
                         const int e = 2 * rr + o;
 #pragma unroll
                         for (int s = 0; s < SL; ++s) {
-                            const double2 kv = e < S::STAGED ? ks[e * 1024 + s * T2]
-                                                             : *reinterpret_cast<const double2 *>(&far[e - S::STAGED][s]);
+                            double2 kv;
+                            if constexpr (S::STAGED) kv = ks[e * 1024 + s * T2];
+                            else kv = *reinterpret_cast<const double2 *>(&kr[e][s]);
                             const double2 v = get_c(y + 4 * s);
                             if (k == 0 && rr == 0) f[o][s] = cx_mul(v, kv);
                             else cx_fma(f[o][s], v, kv);
@@ -290,7 +308,7 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
             }
             tmem_wait_st();
             ct_sync<C>(q);
-            if (t == 0) key.release(n - 1);
+            if (S::STAGED && t == 0) key.release(n - 1);
             if (h < 2) {
                 uint32_t x[32];
                 tmem_ld32_nowait(tm + TT_ACC + 64 * q + 32 * h, x);
@@ -313,7 +331,7 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
     }
     tc_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0) key.drain(a.err);
+    if (S::STAGED && threadIdx.x == 0) key.drain(a.err);
     if (warp == 0) {
         tc_fence_after();
         tmem_dealloc(*slot, 512);

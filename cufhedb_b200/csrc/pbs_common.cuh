@@ -159,7 +159,7 @@ struct BatchPlan {
     BatchPart part[2];
 };
 // pass times (ms) on a B200: 3, 2 and 1 ciphertexts per SM
-constexpr float PBS02_B200_MS[NSHAPES] = {17.15f, 10.89f, 6.20f};
+constexpr float PBS02_B200_MS[NSHAPES] = {16.60f, 10.89f, 5.72f};
 
 inline BatchPlan plan_batch(int B, int num_sms, const int shapes[NSHAPES], const float pass_ms[NSHAPES],
                             const float b200_ms[NSHAPES])

@@ -12,7 +12,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "cufhedb_b200", "csrc")
 SMS, BMAX = 148, 4000
 SHAPES = (3, 2, 1)
-DEFAULT = (17.15, 10.89, 6.20)
+DEFAULT = (16.60, 10.89, 5.72)
 
 PROG = r"""
 #include "pbs_common.cuh"
