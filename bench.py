@@ -47,7 +47,7 @@ WORKLOAD = ("1,024 lvl1 HomNAND gate bootstraps (IKS10 + PBS01 each) over unifor
             "TFHEpp 128-bit params (n=672, N=1024, l=3, Bg=2^6, IKS10 basebit 10 t 2)")
 # DRAM bytes (read + write) of one 1,024-ciphertext PBS launch, from the ncu
 # captures summarised under profiles/ (pbs01_*_batch1024.md)
-TRAFFIC = {"split32": 68_939_264 + 3_732_480, "fp64": 69_385_472 + 3_819_008}
+TRAFFIC = {"split32": 93_320_000 + 6_280_000, "fp64": 148_770_000 + 6_980_000}
 
 
 def parse(argv=None):
@@ -242,6 +242,11 @@ def run_reference(args):
         return
     nthreads = os.cpu_count() or 1
     n = args.batch
+    from oracle.oracle import ref_available
+    if not ref_available():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's TFHEpp is not built (oracle/_ref)"}),
+              flush=True)
+        return
     ref = CpuReference(nthreads)
     ca, cb = ref.inputs(n)
     for _ in range(max(1, args.warmup)):
@@ -516,9 +521,11 @@ def run_ours(args):
 
     # ---- launch-shape autotuning (untimed): one full pass of every shape ----------
     tuned = eng.autotune(levels=(1, 2) if (single and args.filter_rows) else (1,))
-    tune = {f"pbs01_{name}": {"pass_ms_by_shape": tuned[f"pbs01_{name}"],
-                              "ciphertexts_per_cta": eng.launch_shape(1, PREC[name], B)}
-            for name in ("split32", "fp64", "split32tc")}
+    # (the CUDA-core lvl01 kernels run one ciphertext per CTA in every shape)
+    tune = {f"pbs01_{name}": {"pass_ms_by_shape": tuned[f"pbs01_{name}"], "ciphertexts_per_cta": 1}
+            for name in ("split32", "fp64")}
+    tune["pbs01_split32tc"] = {"pass_ms_by_shape": tuned["pbs01_split32tc"],
+                               "ciphertexts_per_cta": eng.launch_shape(1, SPLIT32_TC, B)}
     tune["pbs01_split32"]["stage1_layout"] = eng.launch_layout(B)   # chosen over both split tables
     if single and args.filter_rows:
         tune["pbs02"] = {"pass_ms_by_shape": tuned["pbs02"],
@@ -586,7 +593,8 @@ def run_ours(args):
 
     extra = {}
     cref = None
-    if single and rank == 0 and not args.no_cpu_baseline:
+    from oracle.oracle import ref_available
+    if single and rank == 0 and not args.no_cpu_baseline and ref_available():
         cref = CpuReference(os.cpu_count() or 1)
     if single and rank == 0:
         if args.filter_rows:
