@@ -52,7 +52,6 @@ __device__ __forceinline__ double2 cx_shfl_xor(double2 v, int m)
 {
     return make_double2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
 }
-__device__ __forceinline__ double2 cx_scale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 
 template <typename C> struct cx_real;
 template <> struct cx_real<double2> { using type = double; };

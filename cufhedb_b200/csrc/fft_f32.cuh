@@ -61,18 +61,6 @@ __device__ __forceinline__ float2 fcmul(float2 a, float2 b)
 {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
-// a * conj(b)
-__device__ __forceinline__ float2 fcmulc(float2 a, float2 b)
-{
-    return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(a.y, b.x, -a.x * b.y));
-}
-__device__ __forceinline__ void fcfma(float2 &acc, float2 a, float2 b)
-{
-    acc.x = fmaf(a.x, b.x, acc.x);
-    acc.x = fmaf(-a.y, b.y, acc.x);
-    acc.y = fmaf(a.x, b.y, acc.y);
-    acc.y = fmaf(a.y, b.x, acc.y);
-}
 __device__ __forceinline__ float2 shfl_xor_f2(float2 v, int m)
 {
     return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
@@ -150,32 +138,6 @@ __device__ __forceinline__ float2 w32_const(int j)
     return make_float2(C[j], C[8 - j]);
 }
 
-template <class TT>
-__device__ __forceinline__ void ffft512_fwd(float2 v[16], float2 *xp, const TT &T, int lane)
-{
-    fdft16<1>(v);
-#pragma unroll
-    for (int q2 = 1; q2 < 16; ++q2) v[q2] = fcmul(v[q2], T.tw512[q2 * 32 + lane]);
-    __syncwarp();
-#pragma unroll
-    for (int q2 = 0; q2 < 16; ++q2) xp[xpf_index(lane, q2)] = v[q2];
-    __syncwarp();
-    const int h = lane >> 4, q2 = lane & 15;
-#pragma unroll
-    for (int m1p = 0; m1p < 16; ++m1p) v[m1p] = xp[xpf_index(2 * m1p + h, q2)];
-    fdft16<1>(v);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        float2 send = h ? v[j] : v[8 + j];
-        float2 recv = shfl_xor_f2(send, 16);
-        float2 a = h ? recv : v[j];
-        float2 b = h ? v[8 + j] : recv;
-        float2 t = fcmul(b, T.w32[j + 8 * h]);
-        v[j] = fadd2(a, t);
-        v[8 + j] = fsub2(a, t);
-    }
-}
-
 // a * e^{2 pi i m2 / 64} = a * w^{32 m2} (compile-time constants once unrolled)
 __device__ __forceinline__ float2 cw64(float2 a, int m2)
 {
@@ -188,20 +150,12 @@ __device__ __forceinline__ float2 cw64(float2 a, int m2)
     return make_float2(fmaf(a.x, c, -a.y * sn), fmaf(a.x, sn, a.y * c));
 }
 
-// forward transform of inputs that carry only the per-register part of the
-// twist, v[m2] = (a_m + i a_{m+512}) w^{32 m2} (cw64): the lane's part w^{lane}
-// is applied with the stage-1 twiddles (tw512w, q2 = 0 included), the radix-2
-// twiddles come from constants.  Same output as ffft512_fwd on fully twisted
-// inputs.
-__device__ __forceinline__ void ffft512_fwd_tw_rest(float2 v[16], float2 *xp, const Fft512TablesFold &T, int lane);
-__device__ __forceinline__ void ffft512_fwd_tw(float2 v[16], float2 *xp, const Fft512TablesFold &T, int lane)
-{
-    fdft16<1>(v);
-    ffft512_fwd_tw_rest(v, xp, T, lane);
-}
-
-// everything after the first 16-point DFT: v[q2] = X[q2] of this lane (the
-// tensor-core path computes X on the tensor cores, tc_stage1.cuh)
+// Forward transform of inputs that carry only the per-register part of the
+// twist, v[m2] = (a_m + i a_{m+512}) w^{32 m2} (cw64), after its first 16-point
+// DFT (the tensor-core path computes that on the tensor cores, tc_stage1.cuh):
+// v[q2] = X[q2] of this lane.  The lane's part of the twist w^{lane} is applied
+// with the stage-1 twiddles (tw512w, q2 = 0 included), the radix-2 twiddles come
+// from constants.
 __device__ __forceinline__ void ffft512_fwd_tw_rest(float2 v[16], float2 *xp, const Fft512TablesFold &T, int lane)
 {
 #pragma unroll

@@ -1,5 +1,5 @@
-// Shared-memory key ring of the persistent PBS kernels, without a producer
-// warp.  The bootstrapping key streams through S slots of CHUNK bytes each
+// Shared-memory key rings of the tensor-core PBS kernel; first the one without
+// a producer warp.  The bootstrapping key streams through S slots of CHUNK bytes each
 // (bulk copies completing on one mbarrier per slot).  Thread 0 issues the
 // first S chunks; afterwards the last of the W consumer warps to release a
 // slot refills it with the chunk S positions further on, so every warp of the
