@@ -186,9 +186,14 @@ int launch_pbs01_any(cufhedb_ctx *ctx, Pbs01Args &a, int precision, cudaStream_t
     return CUFHEDB_OK;
 }
 
-// the lvl02 PBS, divided over launches as the context's table makes shortest
+// the lvl02 PBS: large batches one ciphertext per block, others divided over
+// launches as the context's table makes shortest
 int launch_pbs02_any(cufhedb_ctx *ctx, const Pbs02Args &a, cudaStream_t st)
 {
+    if (a.B > PBS02_BLOCKS_MIN * ctx->num_sms) {
+        CK(launch_pbs02_blocks(a, st));
+        return CUFHEDB_OK;
+    }
     const BatchPlan plan = plan_batch(a.B, ctx->num_sms, PBS02_SHAPES, ctx->pbs02_pass_ms, PBS02_B200_MS);
     Pbs02Args p = a;
     for (int k = 0; k < plan.parts; ++k) {

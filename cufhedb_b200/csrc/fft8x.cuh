@@ -163,6 +163,13 @@ struct Fft8xTables {
     C twA0[T];
     C twAs[T];
     C twB1[L];
+    // what the transforms read; a kernel may keep a thread's steps elsewhere
+    __device__ __forceinline__ void stage_a(int t, C &base, C &step) const
+    {
+        base = twA0[t];
+        step = twAs[t];
+    }
+    __device__ __forceinline__ C stage_b(int a) const { return twB1[a]; }
 };
 
 // host: the FP64 tables, computed in long double
@@ -247,13 +254,15 @@ __device__ __forceinline__ int fft8x_xp(int t, int k)
 // v[s] = V(fft8x_freq<T>(t, s)) out.  xp: FFT8X_XP<T>-entry scratch shared
 // by the group; bar: its named barrier.
 // after_first() runs in every thread past the first group barrier.
-template <typename C, int T, class Hook>
-__device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Fft8xTables<C, T> &tab, int t, int bar,
+template <typename C, int T, class Tab, class Hook>
+__device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Tab &tab, int t, int bar,
                                           Hook after_first)
 {
     constexpr int L = T / 8;
     cx_dft8<1>(v);
-    fft8x_twiddle_powers<1>(v, tab.twA0[t], tab.twAs[t]);
+    C base, step;
+    tab.stage_a(t, base, step);
+    fft8x_twiddle_powers<1>(v, base, step);
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < 8; ++k) xp[fft8x_xp<C>(t, k)] = v[k];
@@ -263,7 +272,7 @@ __device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Fft8xTables<C, T>
 #pragma unroll
     for (int b = 0; b < 8; ++b) v[b] = xp[fft8x_xp<C>(a + L * b, k)];
     cx_dft8<1>(v);
-    fft8x_step_powers<1>(v, tab.twB1[a]);
+    fft8x_step_powers<1>(v, tab.stage_b(a));
     // C: the second transpose stays inside the warp (rows t of this warp),
     // but other warps may still be reading these rows from the first one
     group_sync<T>(bar);
@@ -286,16 +295,16 @@ __device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Fft8xTables<C, T>
     }
 }
 
-template <typename C, int T>
-__device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Fft8xTables<C, T> &tab, int t, int bar)
+template <typename C, int T, class Tab>
+__device__ __forceinline__ void fft8x_fwd(C v[8], C *xp, const Tab &tab, int t, int bar)
 {
-    fft8x_fwd<C, T>(v, xp, tab, t, bar, [] {});
+    fft8x_fwd<C, T, Tab>(v, xp, tab, t, bar, [] {});
 }
 
 // inverse: v[s] = V(fft8x_freq<T>(t, s)) in, v[j] = M z_{t + T j} / w^t out
 // (callers multiply by conj(W_32^j) to finish the untwist)
-template <typename C, int T>
-__device__ __forceinline__ void fft8x_inv(C v[8], C *xp, const Fft8xTables<C, T> &tab, int t, int bar)
+template <typename C, int T, class Tab>
+__device__ __forceinline__ void fft8x_inv(C v[8], C *xp, const Tab &tab, int t, int bar)
 {
     constexpr int L = T / 8;
     const int a = t % L, k = t / L;
@@ -319,7 +328,7 @@ __device__ __forceinline__ void fft8x_inv(C v[8], C *xp, const Fft8xTables<C, T>
     __syncwarp();
 #pragma unroll
     for (int q1 = 0; q1 < 8; ++q1) v[q1] = xp[fft8x_xp<C>(t, q1)];
-    fft8x_step_powers<-1>(v, tab.twB1[a]);
+    fft8x_step_powers<-1>(v, tab.stage_b(a));
     cx_dft8<-1>(v);
     group_sync<T>(bar);
 #pragma unroll
@@ -327,7 +336,9 @@ __device__ __forceinline__ void fft8x_inv(C v[8], C *xp, const Fft8xTables<C, T>
     group_sync<T>(bar);
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) v[kk] = xp[fft8x_xp<C>(t, kk)];
-    fft8x_twiddle_powers<-1>(v, tab.twA0[t], tab.twAs[t]);
+    C base, step;
+    tab.stage_a(t, base, step);
+    fft8x_twiddle_powers<-1>(v, base, step);
     cx_dft8<-1>(v);
 }
 

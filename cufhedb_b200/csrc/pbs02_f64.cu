@@ -3,6 +3,9 @@
 // at include/gatebootstrapping.hpp:15-43 with domain lvl0, target lvl2: bbar =
 // 2N - (b >> 20), abar_i = (a_i + 2^19) >> 20).
 //
+// Two kernels: pbs02_team_kernel for batches of a few ciphertexts per SM, and
+// pbs02_block_kernel (below) for larger ones.
+//
 // One persistent CTA per SM holds C = 1 or 2 ciphertexts and four teams of 128
 // threads (8 of the 1,024 points each, fft8x.cuh), 16 warps in all; the teams of
 // a ciphertext (4 or 2) divide every CMux:
@@ -338,6 +341,174 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
     }
 }
 
+// ---- one team per ciphertext and block ---------------------------------------------
+// For batches that fill the SMs many times over: four blocks of four warps per SM,
+// out of step, where the teams of one block wait for one another.  The team does
+// all rows of a CMux itself; its digits' words, its accumulators and its twiddle
+// steps are in tensor memory, the key's values come from L2 into registers, asked
+// for in the middle of the transform before their products.  Shared memory holds
+// the accumulator polynomials and the transpose.  Bound as above, at 67 % of the
+// wavefronts' rate and FP64 at 54 %.  ms per 2,048: 72.4, two per persistent CTA
+// 76.0; key asked for after the transform 79.3, twiddle steps in shared memory
+// 73.1, three blocks of 144 registers 73.6 (four have 128 and spill 68 bytes),
+// two teams per block and three blocks 80.1.
+struct BlockSmem {
+    static constexpr int XP_OFF = 16;
+    static constexpr int ACC_OFF = XP_OFF + FFT8X_XP<T2> * 16;
+    static constexpr int TOTAL = ACC_OFF + 2 * N2 * 8;
+};
+static_assert(BlockSmem::XP_OFF % 16 == 0 && 4 * (BlockSmem::TOTAL + 1024) <= 228 * 1024, "four blocks per SM");
+constexpr uint32_t BT_ACC = 0;       // [output 2][slot 8][re im]
+constexpr uint32_t BT_WORDS = 64;    // [16 words] of the polynomial in work
+constexpr uint32_t BT_TAB = 96;      // twA0, twAs and twB1 of this thread
+constexpr uint32_t BT_COLS = 128;    // of 512 per SM
+
+__device__ __forceinline__ void tmem_ld4_nowait(uint32_t taddr, uint32_t *v)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(taddr)
+                 : "memory");
+}
+struct TmemTables {
+    uint32_t tm;
+    __device__ __forceinline__ void stage_a(int, double2 &a0, double2 &as) const
+    {
+        uint32_t x[8];
+        tmem_ld8_nowait(tm, x);
+        tmem_wait_ld();
+        tmem_landed<8>(x);
+        a0 = get_c(x);
+        as = get_c(x + 4);
+    }
+    __device__ __forceinline__ double2 stage_b(int) const
+    {
+        uint32_t x[4];
+        tmem_ld4_nowait(tm + 8, x);
+        tmem_wait_ld();
+        tmem_landed<4>(x);
+        return get_c(x);
+    }
+};
+
+__global__ void __launch_bounds__(T2, 4) pbs02_block_kernel(Pbs02Args a)
+{
+    using S = BlockSmem;
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint32_t *slot = reinterpret_cast<uint32_t *>(smem);
+    double2 *xp = reinterpret_cast<double2 *>(smem + S::XP_OFF);
+    uint64_t *acc = reinterpret_cast<uint64_t *>(smem + S::ACC_OFF);
+    const int t = threadIdx.x, warp = t >> 5, bar = 1;
+    if (warp == 0) tmem_alloc(slot, BT_COLS);
+    const uint32_t *in = a.in + (size_t)blockIdx.x * (N0 + 1);
+    uint32_t an = in[0];   // the next CMux's mask word, read one CMux ahead
+    {
+        const uint32_t bbar = 2 * N2 - (in[N0] >> 20);
+        for (int m = t; m < N2; m += T2) {
+            acc[m] = 0;
+            acc[N2 + m] = testvec_rot2(a.tv, m, bbar);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tm = *slot + ((32u * warp) << 16);
+    const TmemTables T{tm + BT_TAB};
+    {
+        const Fft1024Tables *src = reinterpret_cast<const Fft1024Tables *>(a.tables);
+        uint32_t x[16];
+        put_c(x, src->twA0[t]);
+        put_c(x + 4, src->twAs[t]);
+        put_c(x + 8, src->twB1[t & 15]);
+        put_c(x + 12, src->twB1[t & 15]);
+        tmem_st16_nowait(tm + BT_TAB, x);
+        tmem_wait_st();
+    }
+
+    // the key: row r, output o, slot s of this thread at [(2 r + o) 1024 + 128 s]
+    const float4 *kg = reinterpret_cast<const float4 *>(a.bk) + t;
+    for (int i = 0; i < N0; ++i, kg += 2 * L2 * 2 * 1024) {
+        const uint32_t ab = (an + (1u << 19)) >> 20;
+        an = in[i + 1];
+        if (ab == 0) continue;
+#pragma unroll 1
+        for (int r = 0; r < 2 * L2; ++r) {
+            uint32_t x[32];
+            uint64_t w[16];
+            if (r % L2 == 0) {
+                digit_words2<true>(w, acc + (r / L2) * N2, ab, t);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    x[2 * j] = (uint32_t)w[j];
+                    x[2 * j + 1] = (uint32_t)(w[j] >> 32);
+                }
+                tmem_st32_nowait(tm + BT_WORDS, x);
+                tmem_wait_st();
+            } else {
+                tmem_ld32_nowait(tm + BT_WORDS, x);
+                tmem_wait_ld();
+                tmem_landed<32>(x);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) w[j] = ((uint64_t)x[2 * j + 1] << 32) | x[2 * j];
+            }
+            double2 v[8];
+            digits2(v, w, r % L2);
+            float4 kv[8];
+            fft8x_fwd<double2, T2>(v, xp, T, t, bar, [&] {
+#pragma unroll
+                for (int s = 0; s < 8; ++s) kv[s] = ldg_here(kg + 2 * r * 1024 + s * T2);
+            });
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                double2 f[8];
+                if (r > 0) {
+                    tmem_ld32_nowait(tm + BT_ACC + 32 * o, x);
+                    tmem_wait_ld();
+                    tmem_landed<32>(x);
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) {
+                        f[s] = get_c(x + 4 * s);
+                        cx_fma(f[s], v[s], *reinterpret_cast<const double2 *>(&kv[s]));
+                    }
+                } else {
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) f[s] = cx_mul(v[s], *reinterpret_cast<const double2 *>(&kv[s]));
+                }
+                if (o == 0) {
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) kv[s] = ldg_here(kg + (2 * r + 1) * 1024 + s * T2);
+                }
+#pragma unroll
+                for (int s = 0; s < 8; ++s) put_c(x + 4 * s, f[s]);
+                tmem_st32_nowait(tm + BT_ACC + 32 * o, x);
+            }
+            tmem_wait_st();
+        }
+#pragma unroll 1
+        for (int o = 0; o < 2; ++o) {
+            uint32_t x[32];
+            tmem_ld32_nowait(tm + BT_ACC + 32 * o, x);
+            tmem_wait_ld();
+            tmem_landed<32>(x);
+            double2 v[8];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) v[s] = get_c(x + 4 * s);
+            fft8x_inv<double2, T2>(v, xp, T, t, bar);
+            add_inverse2(acc + o * N2, v, t);
+        }
+        group_sync<T2>(bar);
+    }
+    uint64_t *o = a.out + (size_t)blockIdx.x * (N2 + 1);
+    for (int m = t; m < N2; m += T2) o[m] = m == 0 ? acc[0] : 0ull - acc[N2 - m];
+    if (t == 0) o[N2] = acc[N2] + a.out_b_add;
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(*slot, BT_COLS);
+    }
+}
+
 template <int C>
 cudaError_t launch_team_t(const Pbs02Args &a, int num_sms, cudaStream_t st)
 {
@@ -374,10 +545,21 @@ cudaError_t launch_pbs02_f64(const Pbs02Args &a, int num_sms, int p, cudaStream_
     return launch_team_t<1>(r, num_sms, st);
 }
 
+// one ciphertext per block, four blocks per SM
+cudaError_t launch_pbs02_blocks(const Pbs02Args &a, cudaStream_t st)
+{
+    if (a.B <= 0) return cudaSuccess;
+    pbs02_block_kernel<<<a.B, T2, BlockSmem::TOTAL, st>>>(a);
+    return cudaGetLastError();
+}
+
 cudaError_t init_pbs02_f64()
 {
-    const cudaError_t e = init_team_t<1>();
-    return e == cudaSuccess ? init_team_t<2>() : e;
+    cudaError_t e = init_team_t<1>();
+    if (e == cudaSuccess) e = init_team_t<2>();
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(pbs02_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BlockSmem::TOTAL);
+    return e;
 }
 
 }  // namespace cfdb

@@ -161,6 +161,13 @@ struct BatchPlan {
 // pass times (ms) on a B200: 3, 2 and 1 ciphertexts per SM
 constexpr float PBS02_B200_MS[NSHAPES] = {16.60f, 10.89f, 5.72f};
 
+// Above this many ciphertexts per SM the one-team blocks (pbs02_f64.cu) run the
+// whole batch: no pass waits for its slowest SM, and four blocks out of step use
+// the pipes better than two ciphertexts' teams; below, the teams' shorter passes
+// win.  ms on 148 SMs, plan -> blocks: 592 21.8 -> 22.2, 888 32.6 -> 32.6,
+// 1,036 38.4 -> 37.7, 1,500 60.1 -> 57.7, 2,048 76.0 -> 72.4, 8,192 304 -> 279.
+constexpr int PBS02_BLOCKS_MIN = 6;
+
 inline BatchPlan plan_batch(int B, int num_sms, const int shapes[NSHAPES], const float pass_ms[NSHAPES],
                             const float b200_ms[NSHAPES])
 {

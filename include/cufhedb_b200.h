@@ -391,7 +391,8 @@ CUFHEDB_API int cufhedb_selftest_wait_timeout(cufhedb_ctx *ctx, uint32_t polls);
  * the least passes x measured pass time is taken, ties to the earlier shape;
  * without measurements all pass times count as equal.  lvl02 and
  * CUFHEDB_SPLIT32_TC launch in the shape (an lvl02 batch may be divided into
- * full passes of one shape and a rest in another where that is shorter);
+ * full passes of one shape and a rest in another where that is shorter, and one
+ * of more than six per SM runs one ciphertext per block);
  * CUFHEDB_FP64 and CUFHEDB_SPLIT32 on the CUDA cores run one ciphertext per
  * block whatever the shape, and their times serve the queue scheduler and the
  * next choice: CUFHEDB_SPLIT32 launches pick the layout of the first transform
@@ -409,7 +410,7 @@ CUFHEDB_API int cufhedb_autotune_pbs02(cufhedb_ctx *ctx, float *ms);
 /* the context's table for a level (1 with FP64 or SPLIT32, 2 with FP64):
  * shapes[3] and pass_ms[3] (either may be NULL); returns 3 */
 CUFHEDB_API int cufhedb_autotune_table(cufhedb_ctx *ctx, int level, int precision, int *shapes, float *pass_ms);
-/* the table's shape (ciphertexts per CTA) for a launch of all B ciphertexts */
+/* the table's shape (ciphertexts per SM) for a launch of all B ciphertexts */
 CUFHEDB_API int cufhedb_launch_shape(cufhedb_ctx *ctx, int level, int precision, int B, int *shape);
 /* the stage-1 layout a CUFHEDB_SPLIT32 launch of B ciphertexts would use now:
  * *tensor_core_stage1 = 1 (tensor cores) or 0 (CUDA cores) */

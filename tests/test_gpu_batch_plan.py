@@ -55,6 +55,23 @@ def test_lvl02_words_equal_across_shapes(lvl2_engines, tv, rows):
     assert all(torch.equal(outs[0], o) for o in outs[1:])
 
 
+def test_lvl02_words_equal_in_large_batches(lvl2_engines):
+    """more than six ciphertexts per SM run one per block: the same words as in
+    small batches, first and last rows, a skipped CMux and the all-zero row"""
+    import torch
+    from cufhedb_b200 import testvec_staircase
+    e = lvl2_engines[0]
+    B = 6 * e.num_sms + 1
+    x = _inputs(B)
+    want = torch.empty(B * (N2 + 1), dtype=torch.int64, device="cuda")
+    e.pbs_lvl02(x, want, testvec_staircase(44))
+    for at in (0, B // 2 - 2, B - 5):
+        got = torch.empty(5 * (N2 + 1), dtype=torch.int64, device="cuda")
+        e.pbs_lvl02(x[at * (N0 + 1): (at + 5) * (N0 + 1)].contiguous(), got, testvec_staircase(44))
+        e.sync()
+        assert torch.equal(got, want[at * (N2 + 1): (at + 5) * (N2 + 1)]), at
+
+
 def _inputs(B):
     """uniform lvl0 words, with mask words that round to rotations 0 and N and
     an all-zero row among them"""
