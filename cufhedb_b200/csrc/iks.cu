@@ -228,28 +228,27 @@ cudaError_t launch_gather(const IksArgs &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-// ---- key-stationary lvl2 -> lvl1 switch (large batches) ------------------------
+// ---- key-stationary lvl2 -> lvl1 switch --------------------------------------------
 // The gather above reads each selected 4,100-byte key row once per ciphertext:
 // 75 GB per 1,024 ciphertexts, served from L2 (the 0.59 GB key stays there).
-// Turned around, each CTA owns 8 output words of 256 ciphertexts and walks
-// the whole key once, staging those 8 words of every key row in shared
-// memory (2.4 GB of L2 reads per 1,024 ciphertexts), and each thread, one
-// ciphertext, subtracts the staged words of the rows its digits select.  The
-// subtractions are the gather's, in the same order per word (ascending i,
-// j), so the results are identical.  Eight words per CTA (129 word blocks)
-// give 28 warps per SM at 1,024 ciphertexts; the staged rows are padded to
-// 48 bytes, so the eight digit values of a quarter-warp's 16-byte reads fall
-// in eight distinct bank groups.
-constexpr int KS_TILE = 256;                          // ciphertexts per CTA, one per thread
+// Turned around, each CTA owns 8 output words of TILE ciphertexts and walks a
+// part of the key, staging those 8 words of every key row in shared memory, and
+// each thread, one ciphertext, subtracts the staged words of the rows its digits
+// select.  Integer sums modulo 2^32: the parts add up to the gather's words.
+// Bound by the shared-memory reads (two of 16 bytes per digit, a wavefront per
+// quarter-warp: 2.4 ms per 1,024) and, per tile, by the staging (about 0.3 ms):
+// so 512 ciphertexts share a tile where there are more than 256, and warps past
+// the batch only stage.  The staged rows are padded to 48 bytes, so the eight
+// digit values of a quarter-warp's 16-byte reads fall in eight distinct bank
+// groups.  The key is divided over CTAs because 129 word blocks a tile fill the
+// SMs unevenly.  ms, whole key per CTA of 256 -> divided, 256 / 512 a tile:
+//   256: 0.98 -> 0.75 / 0.81;  512: 1.92 -> 1.46 / 1.38;  1,024: 3.58 -> 2.86 / 2.70;
+//   2,048: 5.85 -> 5.66 / 5.35;  4,096: 11.8 -> 11.3 / 10.6
 constexpr int KS_WB = 8;                              // output words per CTA
 constexpr int KS_NB = (N1 + 1 + KS_WB - 1) / KS_WB;   // word blocks: 129
-constexpr int KS_IC = 2;                              // input coefficients per staged chunk
 constexpr int KS_DIG = 1 << KS21_BASEBIT;             // digit values 0..7 (row 0: zeros)
-constexpr int KS_ROWS = KS_IC * KS21_T * KS_DIG;      // staged rows per chunk: 160
 constexpr int KS_RW4 = 3;                             // uint4 per staged row: 8 words + 4 pad
 constexpr int KS_P4 = ksk_pitch(N1 + 1) / 4;          // uint4 per key row in HBM: 257
-constexpr int KS_LOADS = KS_IC * KS21_T * (KS_DIG - 1) * (KS_WB / 4);   // uint4 per chunk: 280
-constexpr int KS_PER = (KS_LOADS + KS_TILE - 1) / KS_TILE;              // per thread: 2
 constexpr uint64_t KS_PREC = 1ull << (64 - (1 + KS21_BASEBIT * KS21_T));
 constexpr int KS_SHIFT = 64 - KS21_BASEBIT * KS21_T;                    // the digits' 30 bits
 
@@ -263,12 +262,19 @@ __global__ void ks21_prep_kernel(const uint64_t *__restrict__ in, uint32_t *X, i
     X[idx] = b < B ? (uint32_t)((in[(size_t)b * (N2 + 1) + i] + KS_PREC) >> KS_SHIFT) : 0u;
 }
 
-__global__ void __launch_bounds__(KS_TILE, 4) ks21_kernel(const uint32_t *__restrict__ X, int Bp,
-                                                       const uint4 *__restrict__ ksk, const uint64_t *in,
-                                                       uint32_t *out, int B, uint64_t offset64)
+// TILE ciphertexts per CTA, IC input coefficients per staged chunk; the output
+// holds (0, ..., 0, b') and takes every part's sum
+template <int TILE, int IC>
+__global__ void __launch_bounds__(TILE, 1024 / TILE) ks21_kernel(const uint32_t *__restrict__ X, int Bp,
+                                                                 const uint4 *__restrict__ ksk, uint32_t *out, int B)
 {
+    constexpr int KS_TILE = TILE, KS_IC = IC;
+    constexpr int KS_ROWS = KS_IC * KS21_T * KS_DIG;                               // staged rows per chunk
+    constexpr int KS_LOADS = KS_IC * KS21_T * (KS_DIG - 1) * (KS_WB / 4);          // uint4 per chunk
+    constexpr int KS_PER = (KS_LOADS + KS_TILE - 1) / KS_TILE;                     // per thread
     __shared__ uint4 stage[2][KS_ROWS * KS_RW4];
     const int t = threadIdx.x, s = blockIdx.x, ct = blockIdx.y * KS_TILE + t;
+    const bool live = (ct & ~31) < B;
     // digit-0 rows are zero in both buffers (never written again)
     for (int e = t; e < 2 * KS_IC * KS21_T * KS_RW4; e += KS_TILE) {
         const int buf = e / (KS_IC * KS21_T * KS_RW4), rem = e % (KS_IC * KS21_T * KS_RW4);
@@ -308,15 +314,15 @@ __global__ void __launch_bounds__(KS_TILE, 4) ks21_kernel(const uint32_t *__rest
 #pragma unroll
     for (int k = 0; k < KS_WB; ++k) acc[k] = 0u;
     constexpr int NCHUNK = N2 / KS_IC;
-    load(0);
-    store(0);
+    const int first = NCHUNK * blockIdx.z / gridDim.z, last = NCHUNK * (blockIdx.z + 1) / gridDim.z;
+    load(first);
+    store(first & 1);
     __syncthreads();
 #pragma unroll 1
-    for (int c = 0; c < NCHUNK; ++c) {
-        if (c + 1 < NCHUNK) load(c + 1);
+    for (int c = first; c < last; ++c) {
+        if (c + 1 < last) load(c + 1);
         const uint4 *buf = stage[c & 1];
-#pragma unroll
-        for (int ii = 0; ii < KS_IC; ++ii) {
+        for (int ii = 0; live && ii < KS_IC; ++ii) {
             const uint32_t x = X[(size_t)(c * KS_IC + ii) * Bp + (size_t)blockIdx.y * KS_TILE + t];
 #pragma unroll
             for (int j = 0; j < KS21_T; ++j) {
@@ -332,43 +338,76 @@ __global__ void __launch_bounds__(KS_TILE, 4) ks21_kernel(const uint32_t *__rest
                 }
             }
         }
-        if (c + 1 < NCHUNK) store((c + 1) & 1);
+        if (c + 1 < last) store((c + 1) & 1);
         __syncthreads();
     }
     if (ct >= B) return;
-    const uint32_t bnew = (uint32_t)((in[(size_t)ct * (N2 + 1) + N2] + offset64 + (1ull << 31)) >> 32);
-    uint32_t *o = out + (size_t)ct * (N1 + 1);
+    uint32_t *o = out + (size_t)ct * (N1 + 1) + KS_WB * s;
 #pragma unroll
-    for (int k = 0; k < KS_WB; ++k) {
-        const int w = KS_WB * s + k;
-        if (w < N1) o[w] = acc[k];
-        else if (w == N1) o[w] = acc[k] + bnew;
-    }
+    for (int k = 0; k < KS_WB; ++k)
+        if (KS_WB * s + k <= N1) atomicAdd(o + k, acc[k]);
 }
 
-// batches from this size on take the key-stationary lvl2 -> lvl1 switch
-constexpr int KS21_MIN_BATCH = 512;
+// the key walked in `parts` parts by each word block and tile
+template <int TILE, int IC>
+cudaError_t launch_ks21(const IksArgs &a, uint32_t *X, int Bp, int parts, cudaStream_t st)
+{
+    iks_init_kernel<true, N2, N1 + 1><<<a.B, 256, 0, st>>>(a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const size_t n = (size_t)N2 * Bp;
+    ks21_prep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a.in64, X, a.B, Bp);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    ks21_kernel<TILE, IC><<<dim3(KS_NB, Bp / TILE, parts), TILE, 0, st>>>(X, Bp, reinterpret_cast<const uint4 *>(a.ksk),
+                                                                           a.out, a.B);
+    return cudaGetLastError();
+}
+
+// Batches from KS21_MIN on take the key-stationary switch (ms, gather ->
+// key-stationary: 96 0.39 -> 0.39, 128 0.51 -> 0.47, 200 0.77 -> 0.68, 300 1.14 ->
+// 0.98).  It needs 8 KB of scratch per ciphertext; below KS21_SCRATCH the gather
+// stands in where that is not to be had, and in a stream that is being captured,
+// whose graph then holds no allocation of its own.
+constexpr int KS21_MIN = 128, KS21_SCRATCH = 512;
+
+// done: whether the switch was enqueued
+cudaError_t ks21_key_stationary(const IksArgs &a, bool &done, cudaStream_t st)
+{
+    done = false;
+    if (a.B < KS21_SCRATCH) {
+        cudaStreamCaptureStatus cs;
+        const cudaError_t e = cudaStreamIsCapturing(st, &cs);
+        if (e != cudaSuccess) {
+            cudaGetLastError();   // the gather's launch reports what is wrong with the stream
+            return cudaSuccess;
+        }
+        if (cs != cudaStreamCaptureStatusNone) return cudaSuccess;
+    }
+    const int tile = a.B <= 256 ? 256 : 512, tiles = (a.B + tile - 1) / tile, Bp = tiles * tile;
+    uint32_t *X = nullptr;
+    cudaError_t e = cudaMallocAsync((void **)&X, (size_t)N2 * Bp * sizeof(uint32_t), st);
+    if (e == cudaErrorMemoryAllocation && a.B < KS21_SCRATCH) {
+        cudaGetLastError();   // not this call's failure: the gather needs no scratch
+        return cudaSuccess;
+    }
+    if (e != cudaSuccess) return e;
+    done = true;
+    e = tile == 256 ? launch_ks21<256, 2>(a, X, Bp, 32, st)
+                    : launch_ks21<512, 4>(a, X, Bp, tiles < 4 ? 16 / tiles : 4, st);
+    const cudaError_t ef = cudaFreeAsync(X, st);
+    return e != cudaSuccess ? e : ef;
+}
 
 }  // namespace
 
 cudaError_t launch_iks(const IksArgs &a, int kind, cudaStream_t st)
 {
     if (a.B <= 0) return cudaSuccess;
-    if (kind == 21 && a.B >= KS21_MIN_BATCH) {
-        const int tiles = (a.B + KS_TILE - 1) / KS_TILE, Bp = tiles * KS_TILE;
-        uint32_t *X = nullptr;
-        cudaError_t e = cudaMallocAsync((void **)&X, (size_t)N2 * Bp * sizeof(uint32_t), st);
-        if (e != cudaSuccess) return e;
-        const size_t n = (size_t)N2 * Bp;
-        ks21_prep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a.in64, X, a.B, Bp);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) {
-            ks21_kernel<<<dim3(KS_NB, tiles), KS_TILE, 0, st>>>(X, Bp, reinterpret_cast<const uint4 *>(a.ksk),
-                                                                 a.in64, a.out, a.B, a.offset64);
-            e = cudaGetLastError();
-        }
-        const cudaError_t ef = cudaFreeAsync(X, st);
-        return e != cudaSuccess ? e : ef;
+    if (kind == 21 && a.B >= KS21_MIN) {
+        bool done;
+        const cudaError_t e = ks21_key_stationary(a, done, st);
+        if (e != cudaSuccess || done) return e;
     }
     // one 16-byte word of a padded row per thread: 169 of 192 (lvl0 rows),
     // 257 of 288 (lvl1 rows)

@@ -39,3 +39,34 @@ def test_divided_switch_equals_undivided(ks_engine, kind):
         ks_engine.iks(kind, x[:n].contiguous(), got)
         ks_engine.sync()
         assert torch.equal(got, want[:n]), n
+
+
+@pytest.mark.parametrize("B", [128, 129, 256, 257, 511, 513, 1100, 2100])
+def test_key_stationary_batches_equal_gather(ks_engine, B):
+    """lvl21, batches at the edges of the key-stationary switch's tiles and parts:
+    the words the gather gives (batches of 100); captured, a batch below 512 takes
+    the gather"""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(B)
+    x = torch.randint(-2 ** 63, 2 ** 63 - 1, (B, 2049), generator=g, device="cuda", dtype=torch.int64)
+    x[B // 2] = 0                       # digits of the rounding offset alone
+    x[B - 1] = -1
+    got = torch.full((B, 1025), 7, dtype=torch.int32, device="cuda")
+    want = torch.empty_like(got)
+    ks_engine.iks(21, x, got)
+    for at in range(0, B, 100):
+        n = min(100, B - at)
+        part = torch.empty((n, 1025), dtype=torch.int32, device="cuda")
+        ks_engine.iks(21, x[at: at + n].contiguous(), part)
+        ks_engine.sync()
+        want[at: at + n] = part
+    assert torch.equal(got, want)
+    if B < 512:
+        again = torch.full_like(got, 9)
+        stream = torch.cuda.Stream()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            ks_engine.iks(21, x, again, stream=stream)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(again, want)
