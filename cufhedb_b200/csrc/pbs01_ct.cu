@@ -28,6 +28,8 @@ namespace cfdb {
 
 namespace {
 
+constexpr uint32_t KEY_BYTES = 2 * L1 * 1024 * 16;   // of one CMux
+
 template <class P>
 struct CtSmem {
     static constexpr int TAB_OFF = 64;
@@ -36,12 +38,19 @@ struct CtSmem {
     static constexpr int TOTAL = BUF_OFF + 2 * L1 * P::BUF * (int)sizeof(typename P::V);
 };
 
+// The first `askers` blocks ask the key of the CMux after next into L2, a share
+// each.  A key switch of 5.6 GB has usually run before and left the key in DRAM,
+// whose latency each CMux would then meet; ms with a cold L2, without -> with:
+// split 1: 2.09 -> 1.96, 148: 1.95 -> 1.88, 1,024: 8.58 -> 8.48; FP64 1: 2.72 ->
+// 2.43, 148: 2.52 -> 2.36, 1,024: 12.12 -> 12.11.  Three blocks per SM lose by it
+// (444: 3.85 -> 3.90) and do without.
 template <class P, int NW, int OCC>
-__global__ void __launch_bounds__(32 * NW, OCC) pbs01_ct_kernel(Pbs01Args a)
+__global__ void __launch_bounds__(32 * NW, OCC) pbs01_ct_kernel(Pbs01Args a, uint32_t askers)
 {
     using L = CtSmem<P>;
     using V = typename P::V;
     constexpr int NT = 32 * NW, BUF = P::BUF;
+    constexpr bool ASK = OCC != 3;
     static_assert(NW >= 2 * L1, "one warp per row");
     extern __shared__ __align__(128) unsigned char smem[];
     uint32_t *slot = reinterpret_cast<uint32_t *>(smem);
@@ -75,6 +84,12 @@ __global__ void __launch_bounds__(32 * NW, OCC) pbs01_ct_kernel(Pbs01Args a)
     // the key: row r, slot s, output o of this lane at [1024 r + 64 s + 32 o]
     const float4 *kg = reinterpret_cast<const float4 *>(a.bk) + lane;
     for (int i = 0; i < N0; ++i, kg += 2 * L1 * 1024) {
+        if (ASK && tid == 0 && blockIdx.x < askers && i + 2 < N0) {
+            const uint32_t share = (KEY_BYTES / 16 + askers - 1) / askers * 16, at = blockIdx.x * share;
+            if (at < KEY_BYTES)
+                bulk_prefetch_l2(reinterpret_cast<const unsigned char *>(a.bk) + (size_t)(i + 2) * KEY_BYTES + at,
+                                 min(share, KEY_BYTES - at));
+        }
         const uint32_t ab = (an + (1u << 20)) >> 21;
         an = in[i + 1];
         if (ab == 0) continue;
@@ -119,9 +134,9 @@ __global__ void __launch_bounds__(32 * NW, OCC) pbs01_ct_kernel(Pbs01Args a)
 }
 
 template <class P, int NW, int OCC>
-cudaError_t launch_ct_t(const Pbs01Args &a, cudaStream_t st)
+cudaError_t launch_ct_t(const Pbs01Args &a, int num_sms, cudaStream_t st)
 {
-    pbs01_ct_kernel<P, NW, OCC><<<a.B, 32 * NW, CtSmem<P>::TOTAL, st>>>(a);
+    pbs01_ct_kernel<P, NW, OCC><<<a.B, 32 * NW, CtSmem<P>::TOTAL, st>>>(a, a.B < num_sms ? a.B : num_sms);
     return cudaGetLastError();
 }
 
@@ -145,9 +160,9 @@ cudaError_t init_ct_t()
 cudaError_t launch_pbs01_split(const Pbs01Args &a, int num_sms, cudaStream_t st)
 {
     if (a.B <= 0) return cudaSuccess;
-    if (a.B <= num_sms) return launch_ct_t<SplitPath, 8, 2>(a, st);
-    if (a.B <= 3 * num_sms) return launch_ct_t<SplitPath, 8, 3>(a, st);
-    return launch_ct_t<SplitPath, 8, 4>(a, st);
+    if (a.B <= num_sms) return launch_ct_t<SplitPath, 8, 2>(a, num_sms, st);
+    if (a.B <= 3 * num_sms) return launch_ct_t<SplitPath, 8, 3>(a, num_sms, st);
+    return launch_ct_t<SplitPath, 8, 4>(a, num_sms, st);
 }
 
 // FP64: two CTAs per SM (60 KB and 64 values' registers each).  Alone on its SM a
@@ -158,7 +173,7 @@ cudaError_t launch_pbs01_split(const Pbs01Args &a, int num_sms, cudaStream_t st)
 cudaError_t launch_pbs01_f64(const Pbs01Args &a, int num_sms, cudaStream_t st)
 {
     if (a.B <= 0) return cudaSuccess;
-    return a.B <= num_sms ? launch_ct_t<F64Path, 8, 2>(a, st) : launch_ct_t<F64Path, 6, 2>(a, st);
+    return a.B <= num_sms ? launch_ct_t<F64Path, 8, 2>(a, num_sms, st) : launch_ct_t<F64Path, 6, 2>(a, num_sms, st);
 }
 
 cudaError_t init_pbs01_ct()
