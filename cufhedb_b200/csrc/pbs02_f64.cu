@@ -347,11 +347,12 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
 // all rows of a CMux itself; its digits' words, its accumulators and its twiddle
 // steps are in tensor memory, the key's values come from L2 into registers, asked
 // for in the middle of the transform before their products.  Shared memory holds
-// the accumulator polynomials and the transpose.  Bound as above, at 67 % of the
-// wavefronts' rate and FP64 at 54 %.  ms per 2,048: 72.4, two per persistent CTA
-// 76.0; key asked for after the transform 79.3, twiddle steps in shared memory
-// 73.1, three blocks of 144 registers 73.6 (four have 128 and spill 68 bytes),
-// two teams per block and three blocks 80.1.
+// the accumulator polynomials and the transpose.  Bound by the transposes and
+// FP64 latency: L1 data pipe at 61 %, FP64 at 50 %, issue 53 % (1,184).  ms per
+// 2,048: 72.4, two ciphertexts per persistent CTA 76.0; key asked for after the
+// transform 79.3, twiddle steps in shared memory 73.1, three blocks of 144
+// registers 73.6 (four have 128 and spill 68 bytes), two teams per block and three
+// blocks 80.1.
 struct BlockSmem {
     static constexpr int XP_OFF = 16;
     static constexpr int ACC_OFF = XP_OFF + FFT8X_XP<T2> * 16;
