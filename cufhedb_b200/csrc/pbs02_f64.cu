@@ -209,9 +209,19 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
             const uint32_t ab = valid ? (an + (1u << 19)) >> 20 : 0u;
             an = in[i + 1];
             if (ab == 0) {
-                for (int k = 0; S::STAGED && k < ROUNDS; ++k, ++n) {
-                    key.acquire(n, a.err);
-                    if (t == 0) key.release(n);
+                if constexpr (S::STAGED) {
+                    // One thread takes part in the skipped rounds for its team, which
+                    // does not read them: a warp that waited here as well could be held
+                    // up while the rounds run on, and would then meet the parity of a
+                    // later one.  The others' next acquire follows a ct_sync with this
+                    // thread, and their round cannot be replaced before they release it.
+                    if (t == 0)
+                        for (int k = 0; k < ROUNDS; ++k) {
+                            key.acquire(n + k, a.err);
+                            key.release(n + k);
+                        }
+                    __syncwarp();
+                    n += ROUNDS;
                 }
                 continue;
             }

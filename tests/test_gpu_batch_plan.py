@@ -72,6 +72,27 @@ def test_lvl02_words_equal_in_large_batches(lvl2_engines):
         assert torch.equal(got, want[at * (N2 + 1): (at + 5) * (N2 + 1)]), at
 
 
+@pytest.mark.parametrize("rows", ["all", "pairs", "every other"])
+def test_lvl02_runs_of_skipped_cmuxes(lvl2_engines, rows):
+    """two ciphertexts per SM, three passes and an odd row at the end: rows whose
+    masks all round to rotation 0 (no CMux of theirs runs, so a pair of them passes
+    every round of the key without a transform) and rows between them have the
+    words of one ciphertext per SM"""
+    import torch
+    from cufhedb_b200 import testvec_staircase
+    S = lvl2_engines[0].num_sms
+    B = 4 * S + 3
+    x = _inputs(B).reshape(B, N0 + 1)
+    skip = {"all": slice(0, B), "pairs": [i for i in range(B) if i // 2 % 2], "every other": slice(0, B, 2)}[rows]
+    x[skip, :N0] = (1 << 19) - 1
+    outs = []
+    for e in lvl2_engines[1:3]:
+        outs.append(torch.empty(B * (N2 + 1), dtype=torch.int64, device="cuda"))
+        e.pbs_lvl02(x.reshape(-1), outs[-1], testvec_staircase(44))
+        e.sync()
+    assert torch.equal(*outs)
+
+
 def _inputs(B):
     """uniform lvl0 words, with mask words that round to rotations 0 and N and
     an all-zero row among them"""
