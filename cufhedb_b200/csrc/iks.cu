@@ -213,10 +213,24 @@ int iks_parts(int B)
     return p < NIN / 16 ? p : NIN / 16;
 }
 
+// Whether the output shares bytes with an input, as in a switch of one row in
+// place.  The divided forms write the output before they have read the input, so
+// these calls take the undivided gather, which reads a row first.
+template <int NIN, int NOUT>
+bool in_place(const IksArgs &a)
+{
+    const uintptr_t o = (uintptr_t)a.out, oe = o + (size_t)a.B * NOUT * sizeof(uint32_t);
+    auto meets = [&](const void *in, size_t word) {
+        const uintptr_t i = (uintptr_t)in;
+        return in && i < oe && o < i + (size_t)a.B * (NIN + 1) * word;
+    };
+    return meets(a.in32, 4) || meets(a.in32b, 4) || meets(a.in64, 8);
+}
+
 template <int NT, bool WIDE, int NIN, int BASEBIT, int TT, int NOUT>
 cudaError_t launch_gather(const IksArgs &a, cudaStream_t st)
 {
-    const int parts = iks_parts<NIN>(a.B);
+    const int parts = in_place<NIN, NOUT>(a) ? 1 : iks_parts<NIN>(a.B);
     if (parts == 1) {
         iks_kernel<NT, WIDE, NIN, BASEBIT, TT, NOUT, false><<<a.B, NT, 0, st>>>(a);
         return cudaGetLastError();
@@ -404,7 +418,7 @@ cudaError_t ks21_key_stationary(const IksArgs &a, bool &done, cudaStream_t st)
 cudaError_t launch_iks(const IksArgs &a, int kind, cudaStream_t st)
 {
     if (a.B <= 0) return cudaSuccess;
-    if (kind == 21 && a.B >= KS21_MIN) {
+    if (kind == 21 && a.B >= KS21_MIN && !in_place<N2, N1 + 1>(a)) {
         bool done;
         const cudaError_t e = ks21_key_stationary(a, done, st);
         if (e != cudaSuccess || done) return e;

@@ -70,3 +70,21 @@ def test_key_stationary_batches_equal_gather(ks_engine, B):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(again, want)
+
+
+@pytest.mark.parametrize("kind", [10, 20, 21])
+def test_one_row_switches_in_place(ks_engine, kind):
+    """the output over the row that it is made from, at its start and further in"""
+    import torch
+    win, wout = WIDTH[kind]
+    g = torch.Generator(device="cuda").manual_seed(100 + kind)
+    dt, lim = (torch.int32, 2 ** 31) if kind == 10 else (torch.int64, 2 ** 63)
+    x = torch.randint(-lim, lim - 1, (win,), generator=g, device="cuda", dtype=dt)
+    want = torch.empty(wout, dtype=torch.int32, device="cuda")
+    ks_engine.iks(kind, x, want)
+    for at in (0, 300):
+        row = x.clone()
+        got = row.view(torch.int32)[at: at + wout]
+        ks_engine.iks(kind, row, got)
+        ks_engine.sync()
+        assert torch.equal(got, want), at
