@@ -236,6 +236,7 @@ int gate_enqueue(cufhedb_ctx *ctx, int gate, const uint32_t *ca, const uint32_t 
     k.out = mid;
     k.ksk = ctx->ksk[0];
     k.B = B;
+    k.num_sms = ctx->num_sms;
     cudaError_t e = launch_iks(k, 10, st);
     cufhedb_testvec tv{CUFHEDB_TV_CONST, 0, 1u << 29, nullptr};
     int rc = (e == cudaSuccess) ? pbs01_enqueue(ctx, mid, out, B, &tv, precision, st) : cuda_fail(e, "iks10");
@@ -310,6 +311,7 @@ int iks_run(cufhedb_ctx *ctx, int kind, const void *in, const uint32_t *in_b, in
     k.out = out;
     k.ksk = ctx->ksk[slot];
     k.B = B;
+    k.num_sms = ctx->num_sms;
     CK(launch_iks(k, kind, st));
     return CUFHEDB_OK;
 }
@@ -333,6 +335,7 @@ int gate_enqueue_into(cufhedb_ctx *ctx, int gate, const uint32_t *ca, const uint
     k.out = scratch_lvl0;
     k.ksk = ctx->ksk[0];
     k.B = B;
+    k.num_sms = ctx->num_sms;
     CK(launch_iks(k, 10, st));
     cufhedb_testvec tv{CUFHEDB_TV_CONST, 0, 1u << 29, nullptr};
     return pbs01_enqueue(ctx, scratch_lvl0, out, B, &tv, precision, st);
@@ -1136,6 +1139,7 @@ int cufhedb_iks(cufhedb_ctx *ctx, int kind, const void *in, uint32_t *out, int B
     a.out = out;
     a.ksk = ctx->ksk[slot];
     a.B = B;
+    a.num_sms = ctx->num_sms;
     CK(launch_iks(a, kind, (cudaStream_t)stream));
     return CUFHEDB_OK;
 }

@@ -194,23 +194,33 @@ __global__ void __launch_bounds__(NT) iks_kernel(IksArgs a)
 
 // Parts per ciphertext.  One CTA keeps 8 rows (24 KB) in flight and takes 0.57 ms
 // (lvl10) over its 2,048 rows however empty the GPU is, so a batch is divided
-// into about IKS_CTAS CTAs, of at least 16 input coefficients each; many short
-// CTAs also leave no half-empty last wave (IKS_WAVE of them are resident).
-// The undivided form is left where it is the faster one: a batch that nearly
-// fills one wave, or several, walks the key in step and shares its rows in L2.
-// Measured, ms undivided -> divided (lvl10 / lvl20 / lvl21):
-//   1: 0.213 -> 0.025 / 0.395 -> 0.026 / 3.42 -> 0.037
-//   148: 0.574 -> 0.142 / 1.08 -> 0.262 / 2.55 -> 0.58
-//   592: 0.589 -> 0.396 / 1.11 -> 0.768 / 2.29 -> 2.23
-//   700: 0.597 -> 0.489 / 1.14 -> 0.977;  1,024: 0.602 -> 0.663 / 1.20 -> 1.48
-//   1,500: 1.25 -> 0.957 / 2.31 -> 1.95;  2,048: 1.25 -> 1.29 / 2.38 -> 2.74
-constexpr int IKS_CTAS = 9472, IKS_WAVE = 1184;
-template <int NIN>
-int iks_parts(int B)
+// into about 64 CTAs per SM, of at least 16 input coefficients each.  The
+// undivided form is left where it is the faster one: a batch that nearly fills one
+// wave of resident CTAs (10 per SM for lvl10, of 32 registers a thread, and 8 for
+// lvl20, of 34), or more than one and a half, walks the key in step and shares its
+// rows in L2.  So a batch is divided up to FEW ciphertexts per SM, and from one
+// wave to TAIL per SM, where the undivided form runs a second, nearly empty one.
+// ms on 148 SMs, undivided -> divided (lvl21: batches of 128 and more come here only
+// without scratch):
+//   lvl10   1: 0.213 -> 0.025;  148: 0.574 -> 0.142;  592: 0.589 -> 0.396;
+//     850: 0.600 -> 0.545;  950: 0.615 -> 0.636;  1,300: 0.693 -> 0.813;
+//     1,480: 0.717 -> 0.934;  1,481: 1.25 -> 0.930;  1,850: 1.27 -> 1.13;
+//     2,072: 1.30 -> 1.32
+//   lvl20   1: 0.395 -> 0.026;  148: 1.08 -> 0.262;  592: 1.11 -> 0.768;
+//     750: 1.14 -> 1.05;  850: 1.16 -> 1.18;  1,100: 1.27 -> 1.49;  1,184: 1.30 -> 1.33;
+//     1,185: 2.33 -> 1.40;  1,850: 2.45 -> 2.37;  1,900: 2.47 -> 2.56
+//   lvl21   1: 3.42 -> 0.037;  148: 2.55 -> 0.58;  511: 2.22 -> 1.94
+struct GatherRule {
+    double few, wave, tail;   // ciphertexts per SM
+};
+constexpr GatherRule IKS10_RULE{5.75, 10.0, 12.8}, IKS20_RULE{5.4, 8.0, 12.5};
+
+inline int iks_parts(int B, int num_sms, const GatherRule &r, int max_parts)
 {
-    if ((B > 850 && B <= IKS_WAVE) || B > 1900) return 1;
-    const int p = (IKS_CTAS + B - 1) / B;
-    return p < NIN / 16 ? p : NIN / 16;
+    const double per_sm = (double)B / num_sms;
+    if (per_sm > r.tail || (per_sm > r.few && per_sm <= r.wave)) return 1;
+    const int p = (int)((64ll * num_sms + B - 1) / B);
+    return p < max_parts ? p : max_parts;
 }
 
 // Whether the output shares bytes with an input, as in a switch of one row in
@@ -228,9 +238,9 @@ bool in_place(const IksArgs &a)
 }
 
 template <int NT, bool WIDE, int NIN, int BASEBIT, int TT, int NOUT>
-cudaError_t launch_gather(const IksArgs &a, cudaStream_t st)
+cudaError_t launch_gather(const IksArgs &a, const GatherRule &rule, cudaStream_t st)
 {
-    const int parts = in_place<NIN, NOUT>(a) ? 1 : iks_parts<NIN>(a.B);
+    const int parts = in_place<NIN, NOUT>(a) ? 1 : iks_parts(a.B, a.num_sms, rule, NIN / 16);
     if (parts == 1) {
         iks_kernel<NT, WIDE, NIN, BASEBIT, TT, NOUT, false><<<a.B, NT, 0, st>>>(a);
         return cudaGetLastError();
@@ -425,9 +435,9 @@ cudaError_t launch_iks(const IksArgs &a, int kind, cudaStream_t st)
     }
     // one 16-byte word of a padded row per thread: 169 of 192 (lvl0 rows),
     // 257 of 288 (lvl1 rows)
-    if (kind == 10) return launch_gather<192, false, N1, KS10_BASEBIT, KS10_T, N0 + 1>(a, st);
-    if (kind == 20) return launch_gather<192, true, N2, KS20_BASEBIT, KS20_T, N0 + 1>(a, st);
-    if (kind == 21) return launch_gather<288, true, N2, KS21_BASEBIT, KS21_T, N1 + 1>(a, st);
+    if (kind == 10) return launch_gather<192, false, N1, KS10_BASEBIT, KS10_T, N0 + 1>(a, IKS10_RULE, st);
+    if (kind == 20) return launch_gather<192, true, N2, KS20_BASEBIT, KS20_T, N0 + 1>(a, IKS20_RULE, st);
+    if (kind == 21) return launch_gather<288, true, N2, KS21_BASEBIT, KS21_T, N1 + 1>(a, IKS20_RULE, st);
     return cudaErrorInvalidValue;
 }
 

@@ -16,6 +16,7 @@ struct IksArgs {
     uint32_t *out;
     const uint32_t *ksk;   // rows of ksk_pitch(out width) words, 16-byte aligned
     int B;
+    int num_sms;
 };
 
 cudaError_t launch_iks(const IksArgs &a, int kind, cudaStream_t st);

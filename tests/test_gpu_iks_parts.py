@@ -88,3 +88,25 @@ def test_one_row_switches_in_place(ks_engine, kind):
         ks_engine.iks(kind, row, got)
         ks_engine.sync()
         assert torch.equal(got, want), at
+
+
+@pytest.mark.parametrize("kind", [10, 20])
+def test_switch_words_at_the_edges_of_one_wave(ks_engine, kind):
+    """batches on both sides of every line of the rule (few, one wave, its tail)
+    against the same rows in batches of 100, which are divided finely"""
+    import torch
+    win, wout = WIDTH[kind]
+    S = ks_engine.num_sms
+    few, wave, tail = {10: (5.75, 10, 12.8), 20: (5.4, 8, 12.5)}[kind]
+    sizes = [int(x * S) + k for x in (few, wave, tail) for k in (0, 1)]
+    g = torch.Generator(device="cuda").manual_seed(200 + kind)
+    dt, lim = (torch.int32, 2 ** 31) if kind == 10 else (torch.int64, 2 ** 63)
+    x = torch.randint(-lim, lim - 1, (max(sizes), win), generator=g, device="cuda", dtype=dt)
+    want = torch.empty(len(x), wout, dtype=torch.int32, device="cuda")
+    for at in range(0, len(x), 100):
+        ks_engine.iks(kind, x[at: at + 100], want[at: at + 100])
+    for n in sizes:
+        got = torch.full((n, wout), 0x55555555, dtype=torch.int32, device="cuda")
+        ks_engine.iks(kind, x[:n], got)
+        ks_engine.sync()
+        assert torch.equal(got, want[:n]), n
