@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(32 * NW, OCC) pbs01_ct_kernel(Pbs01Args a, uin
                        [&](int m, uint32_t x) { acc[m] += x; });
         __syncthreads();
     }
+    __syncthreads();   // a row may be bootstrapped over itself, and skipped CMuxes have no barrier
     uint32_t *o = a.out + (size_t)ct * (N1 + 1);
     for (int j = tid; j < N1; j += NT) o[j] = j == 0 ? acc[0] : (uint32_t)(0u - acc[N1 - j]);
     if (tid == 0) o[N1] = acc[N1] + a.out_b_add;

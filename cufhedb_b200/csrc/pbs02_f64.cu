@@ -335,6 +335,7 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
             }
             ct_sync<C>(q);
         }
+        ct_sync<C>(q);   // a row may be bootstrapped over itself, and skipped CMuxes have no barrier
         if (valid) {
             uint64_t *o = a.out + (size_t)ct * (N2 + 1);
             for (int m = t + h * T2; m < N2; m += TPC * T2) o[m] = m == 0 ? acc[0] : 0ull - acc[N2 - m];
@@ -509,6 +510,7 @@ __global__ void __launch_bounds__(T2, 4) pbs02_block_kernel(Pbs02Args a)
         }
         group_sync<T2>(bar);
     }
+    group_sync<T2>(bar);   // skipped CMuxes have no barrier
     uint64_t *o = a.out + (size_t)blockIdx.x * (N2 + 1);
     for (int m = t; m < N2; m += T2) o[m] = m == 0 ? acc[0] : 0ull - acc[N2 - m];
     if (t == 0) o[N2] = acc[N2] + a.out_b_add;

@@ -93,6 +93,36 @@ def test_lvl02_runs_of_skipped_cmuxes(lvl2_engines, rows):
     assert torch.equal(*outs)
 
 
+def test_one_row_bootstraps_in_place(lvl2_engines):
+    """the output over the row that it is made from, whose last CMuxes (or all) are
+    skipped: no barrier stands between them and the output"""
+    import torch
+    from cufhedb_b200 import FP64, GEN_BK01, SPLIT32, Engine, testvec_staircase
+    rows = _inputs(64).reshape(64, N0 + 1)[8:24].clone()
+    for k, row in enumerate(rows):
+        row[N0 - 42 * k: N0] = (1 << 19) - 1
+    with Engine(0) as eng:
+        eng.keygen(SEED, GEN_BK01)
+        for prec in (SPLIT32, FP64):
+            for row in rows:
+                want = torch.empty(N1 + 1, dtype=torch.int32, device="cuda")
+                eng.pbs_lvl01(row, want, testvec_staircase(20), prec)
+                buf = torch.zeros_like(want)
+                buf[: N0 + 1] = row
+                eng.pbs_lvl01(buf[: N0 + 1], buf, testvec_staircase(20), prec)
+                eng.sync()
+                assert torch.equal(buf, want)
+    for e in lvl2_engines:
+        for row in rows[::5]:
+            want = torch.empty(N2 + 1, dtype=torch.int64, device="cuda")
+            e.pbs_lvl02(row, want, testvec_staircase(44))
+            buf = torch.zeros_like(want)
+            buf.view(torch.int32)[: N0 + 1] = row
+            e.pbs_lvl02(buf.view(torch.int32)[: N0 + 1], buf, testvec_staircase(44))
+            e.sync()
+            assert torch.equal(buf, want)
+
+
 def _inputs(B):
     """uniform lvl0 words, with mask words that round to rotations 0 and N and
     an all-zero row among them"""
