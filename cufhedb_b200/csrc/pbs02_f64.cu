@@ -60,6 +60,7 @@ struct TeamShape {
     // registers
     static constexpr bool STAGED = C == 2;
     static constexpr uint32_t BYTES = STAGED ? CHUNKS * CHUNK : 0;
+    using Key = RoundKey<BYTES, TEAMS>;
     static constexpr int KEY_OFF = 128;
     static constexpr int TAB_OFF = KEY_OFF + (int)BYTES;
     static constexpr int XP_OFF = TAB_OFF + ((int)sizeof(Fft1024Tables) + 127) / 128 * 128;
@@ -68,59 +69,6 @@ struct TeamShape {
     static constexpr int ACC_BYTES = 2 * N2 * 8;
     static constexpr int TOTAL = ACC_OFF + C * ACC_BYTES;
     static_assert(TOTAL <= 227 * 1024, "shared memory budget");
-};
-
-// The key of one round in shared memory: one bulk copy, issued by the last
-// team to release the round before.  Waits are bounded; after one gives up
-// nothing is waited for or issued any more.
-template <int C>
-struct RoundKey {
-    using S = TeamShape<C>;
-    unsigned char *head;    // mbarrier, release count, issue count, abort flag
-    unsigned char *stage;
-    const unsigned char *src;
-    uint32_t total;         // rounds this block consumes
-
-    __device__ __forceinline__ uint64_t *full() const { return reinterpret_cast<uint64_t *>(head); }
-    __device__ __forceinline__ int *count() const { return reinterpret_cast<int *>(head + 8); }
-    __device__ __forceinline__ int *issued() const { return reinterpret_cast<int *>(head + 12); }
-    __device__ __forceinline__ volatile int *abort_flag() const { return reinterpret_cast<volatile int *>(head + 16); }
-
-    __device__ __forceinline__ void init()
-    {
-        mbar_init(full(), 1);
-        *count() = 0;
-        *issued() = 0;
-        *abort_flag() = 0;
-        fence_barrier_init();
-    }
-    __device__ __forceinline__ void issue(uint32_t n)
-    {
-        ++*issued();
-        mbar_arrive_expect_tx(full(), S::BYTES);
-        bulk_g2s(stage, src + (size_t)(n % (N0 * S::ROUNDS)) * S::CHUNKS * S::CHUNK, S::BYTES, full());
-    }
-    __device__ __forceinline__ void acquire(uint32_t n, int *err)
-    {
-        if (*abort_flag() == 0 && !mbar_wait(full(), n & 1)) {
-            report_error(err, DEV_TIMEOUT_FULL);
-            *abort_flag() = 1;
-        }
-    }
-    // one thread per team, after the team's last read of round n
-    __device__ __forceinline__ void release(uint32_t n)
-    {
-        if (ring_release(count(), n, TEAMS) && n + 1 < total && *abort_flag() == 0) {
-            fence_proxy_async_smem();
-            issue(n + 1);
-        }
-    }
-    // one thread, at the end: nothing may still be landing
-    __device__ __forceinline__ void drain(int *err)
-    {
-        if (*abort_flag() != 0 && *issued() > 0 && !mbar_wait(full(), (uint32_t)(*issued() - 1) & 1))
-            report_error(err, DEV_TIMEOUT_DRAIN);
-    }
 };
 
 // tensor-memory columns (of every lane; a double is two columns)
@@ -168,8 +116,8 @@ __global__ void __launch_bounds__(TEAMS * T2, 1) pbs02_team_kernel(Pbs02Args a)
     extern __shared__ __align__(128) unsigned char smem[];
     Fft1024Tables *T = reinterpret_cast<Fft1024Tables *>(smem + S::TAB_OFF);
     const int ngroups = (a.B + C - 1) / C;
-    RoundKey<C> key{smem, smem + S::KEY_OFF, reinterpret_cast<const unsigned char *>(a.bk),
-                    (uint32_t)groups_of_block(ngroups, blockIdx.x, gridDim.x) * N0 * ROUNDS};
+    typename S::Key key{smem, smem + S::KEY_OFF, reinterpret_cast<const unsigned char *>(a.bk), N0 * ROUNDS,
+                        (uint32_t)groups_of_block(ngroups, blockIdx.x, gridDim.x) * N0 * ROUNDS};
     uint32_t *slot = reinterpret_cast<uint32_t *>(smem + 64);
 
     const int warp = threadIdx.x >> 5;

@@ -1,5 +1,7 @@
-// Shared-memory key rings of the tensor-core PBS kernel; first the one without
-// a producer warp.  The bootstrapping key streams through S slots of CHUNK bytes each
+// Shared-memory key feeds: the rings of the tensor-core lvl01 kernel, and the
+// staged round of the lvl02 team kernel (RoundKey, at the end).
+//
+// First the ring without a producer warp.  The bootstrapping key streams through S slots of CHUNK bytes each
 // (bulk copies completing on one mbarrier per slot).  Thread 0 issues the
 // first S chunks; afterwards the last of the W consumer warps to release a
 // slot refills it with the chunk S positions further on, so every warp of the
@@ -160,6 +162,68 @@ struct ProducerRing {
     {
         __syncwarp();
         if (lane == 0) mbar_arrive(&h->empty[c % S]);
+    }
+};
+
+// One stage of BYTES that `RELEASERS` teams read together, round after round: one
+// bulk copy per round, issued by the last team to release the round before.
+// `head` (HEAD_BYTES, 8-byte aligned): the mbarrier, the release count, the rounds
+// issued, the abort flag.  Waits are bounded; after one gives up nothing is waited
+// for or issued any more.
+//
+// The barrier has one phase per round and is waited for by its parity, so a
+// thread may call acquire(n) only while its team has not released round n, and
+// only after the team is past round n - 1: round n + 1 cannot then land before it
+// has looked.  Threads that do not read a round leave it to the releasing one.
+template <uint32_t BYTES, int RELEASERS>
+struct RoundKey {
+    static constexpr int HEAD_BYTES = 24;
+    unsigned char *head;
+    unsigned char *stage;
+    const unsigned char *src;      // the key: `per_pass` rounds
+    uint32_t per_pass;
+    uint32_t total;                // rounds this block consumes
+    uint32_t limit = WAIT_LIMIT;   // polls per bounded wait
+
+    __device__ __forceinline__ uint64_t *full() const { return reinterpret_cast<uint64_t *>(head); }
+    __device__ __forceinline__ int *count() const { return reinterpret_cast<int *>(head + 8); }
+    __device__ __forceinline__ int *issued() const { return reinterpret_cast<int *>(head + 12); }
+    __device__ __forceinline__ volatile int *abort_flag() const { return reinterpret_cast<volatile int *>(head + 16); }
+
+    __device__ __forceinline__ void init()
+    {
+        mbar_init(full(), 1);
+        *count() = 0;
+        *issued() = 0;
+        *abort_flag() = 0;
+        fence_barrier_init();
+    }
+    __device__ __forceinline__ void issue(uint32_t n)
+    {
+        ++*issued();
+        mbar_arrive_expect_tx(full(), BYTES);
+        bulk_g2s(stage, src + (size_t)(n % per_pass) * BYTES, BYTES, full());
+    }
+    __device__ __forceinline__ void acquire(uint32_t n, int *err)
+    {
+        if (*abort_flag() == 0 && !mbar_wait(full(), n & 1, limit)) {
+            report_error(err, DEV_TIMEOUT_FULL);
+            *abort_flag() = 1;
+        }
+    }
+    // one thread per team, after the team's last read of round n
+    __device__ __forceinline__ void release(uint32_t n)
+    {
+        if (ring_release(count(), n, RELEASERS) && n + 1 < total && *abort_flag() == 0) {
+            fence_proxy_async_smem();
+            issue(n + 1);
+        }
+    }
+    // one thread, at the end: nothing may still be landing
+    __device__ __forceinline__ void drain(int *err)
+    {
+        if (*abort_flag() != 0 && *issued() > 0 && !mbar_wait(full(), (uint32_t)(*issued() - 1) & 1, limit))
+            report_error(err, DEV_TIMEOUT_DRAIN);
     }
 };
 

@@ -380,9 +380,10 @@ CUFHEDB_API int cufhedb_compare_host_multi(cufhedb_ctx *const *ctxs, int nctx, i
 
 /* Self-test of the kernels' bounded waits (no counterpart in the reference,
  * which has none): one block waits `polls` times (1 .. 2^20) for a key-ring
- * chunk that is never issued, gives up, records the failure and returns.
- * Returns what cufhedb_sync then reports: CUFHEDB_ERR_DEVICE with the wait's
- * code when the path works; the context stays usable afterwards. */
+ * chunk that is never issued, gives up, records the failure and returns; then
+ * another does so for a staged round of the lvl02 key.  Returns what
+ * cufhedb_sync reports after each: CUFHEDB_ERR_DEVICE with the wait's code when
+ * both do; the context stays usable afterwards. */
 CUFHEDB_API int cufhedb_selftest_wait_timeout(cufhedb_ctx *ctx, uint32_t polls);
 
 /* ---- launch-shape autotuner --------------------------------------------------- */
