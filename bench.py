@@ -529,7 +529,8 @@ def run_ours(args):
     tune["pbs01_split32"]["stage1_layout"] = eng.launch_layout(B)   # chosen over both split tables
     if single and args.filter_rows:
         tune["pbs02"] = {"pass_ms_by_shape": tuned["pbs02"],
-                         "ciphertexts_per_cta_filter": eng.launch_shape(2, FP64, args.filter_rows)}
+                         # (a CTA holds one or two; large batches run one per CTA)
+                         "ciphertexts_per_cta_filter": min(2, eng.launch_shape(2, FP64, args.filter_rows))}
 
     # ---- the timed gate steps, headline path then the other path ----------------
     res = {}

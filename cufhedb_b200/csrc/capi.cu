@@ -190,7 +190,7 @@ int launch_pbs01_any(cufhedb_ctx *ctx, Pbs01Args &a, int precision, cudaStream_t
 // launches as the context's table makes shortest
 int launch_pbs02_any(cufhedb_ctx *ctx, const Pbs02Args &a, cudaStream_t st)
 {
-    if (a.B > PBS02_BLOCKS_MIN * ctx->num_sms) {
+    if (pbs02_in_blocks(a.B, ctx->num_sms)) {
         CK(launch_pbs02_blocks(a, st));
         return CUFHEDB_OK;
     }
@@ -1019,8 +1019,12 @@ int cufhedb_launch_shape(cufhedb_ctx *ctx, int level, int precision, int B, int 
     NEED(t != nullptr && B > 0, "bad level, precision or batch");
     if (level == 1 && precision == CUFHEDB_SPLIT32)
         *shape = pbs01_split_choose(B, ctx->num_sms, t, ctx->pbs01_pass_ms[CUFHEDB_SPLIT32_TC]).w;
-    else
-        *shape = level == 1 ? pbs01_choose_w(B, ctx->num_sms, t) : pbs02_choose_p(B, ctx->num_sms, t);
+    else if (level == 1)
+        *shape = pbs01_choose_w(B, ctx->num_sms, t);
+    else   // as launch_pbs02_any
+        *shape = pbs02_in_blocks(B, ctx->num_sms)
+                     ? 1
+                     : plan_batch(B, ctx->num_sms, PBS02_SHAPES, t, PBS02_B200_MS).part[0].w;
     return CUFHEDB_OK;
 }
 

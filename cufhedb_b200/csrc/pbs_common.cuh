@@ -167,6 +167,7 @@ constexpr float PBS02_B200_MS[NSHAPES] = {16.60f, 10.89f, 5.72f};
 // win.  ms on 148 SMs, plan -> blocks: 592 21.8 -> 22.2, 888 32.6 -> 32.6,
 // 1,036 38.4 -> 37.7, 1,500 60.1 -> 57.7, 2,048 76.0 -> 72.4, 8,192 304 -> 279.
 constexpr int PBS02_BLOCKS_MIN = 6;
+inline bool pbs02_in_blocks(int B, int num_sms) { return B > PBS02_BLOCKS_MIN * num_sms; }
 
 inline BatchPlan plan_batch(int B, int num_sms, const int shapes[NSHAPES], const float pass_ms[NSHAPES],
                             const float b200_ms[NSHAPES])

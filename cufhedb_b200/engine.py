@@ -153,14 +153,15 @@ class Engine:
 
     def autotune_pbs01(self, precision: int = _lib.FP64):
         """time one full pass of each lvl01 launch shape (7, 8 and 4
-        ciphertexts per CTA); later launches pick the shape with the least
-        passes x pass time for their batch.  Returns (ms7, ms8)."""
+        ciphertexts per SM); later launches pick the shape, or the split path's
+        stage-1 layout, with the least passes x pass time for their batch.
+        Returns (ms7, ms8)."""
         a, b = C.c_float(0.0), C.c_float(0.0)
         check(self.lib.cufhedb_autotune_pbs01(self.ctx, precision, C.byref(a), C.byref(b)))
         return a.value, b.value
 
     def autotune_pbs02(self):
-        """time one full pass of each lvl02 launch shape (3, 2, 1 per CTA);
+        """time one full pass of each lvl02 launch shape (3, 2, 1 per SM);
         returns the three pass times"""
         ms = (C.c_float * 3)()
         check(self.lib.cufhedb_autotune_pbs02(self.ctx, ms))
@@ -175,7 +176,9 @@ class Engine:
         return {int(w): float(t) for w, t in zip(shapes, ms)}
 
     def launch_shape(self, level: int, precision: int, B: int) -> int:
-        """ciphertexts per CTA a launch of B bootstraps would use now"""
+        """ciphertexts per SM in a pass of a launch of B bootstraps: lvl02 as it
+        would run now (1 where it runs one per block); lvl01 the table's choice,
+        in which the tensor-core kernel launches"""
         w = C.c_int(0)
         check(self.lib.cufhedb_launch_shape(self.ctx, level, precision, B, C.byref(w)))
         return w.value

@@ -390,7 +390,7 @@ CUFHEDB_API int cufhedb_selftest_wait_timeout(cufhedb_ctx *ctx, uint32_t polls);
 /* Launch shapes are ciphertexts per SM in a pass: lvl01 7, 8 and 4, lvl02 3, 2
  * and 1.  A batch of B takes ceil(ceil(B / shape) / SMs) passes; the shape with
  * the least passes x measured pass time is taken, ties to the earlier shape;
- * without measurements all pass times count as equal.  lvl02 and
+ * without measurements all pass times count as equal (lvl02: as a B200's).  lvl02 and
  * CUFHEDB_SPLIT32_TC launch in the shape (an lvl02 batch may be divided into
  * full passes of one shape and a rest in another where that is shorter, and one
  * of more than six per SM runs one ciphertext per block);
@@ -411,7 +411,10 @@ CUFHEDB_API int cufhedb_autotune_pbs02(cufhedb_ctx *ctx, float *ms);
 /* the context's table for a level (1 with FP64 or SPLIT32, 2 with FP64):
  * shapes[3] and pass_ms[3] (either may be NULL); returns 3 */
 CUFHEDB_API int cufhedb_autotune_table(cufhedb_ctx *ctx, int level, int precision, int *shapes, float *pass_ms);
-/* the table's shape (ciphertexts per SM) for a launch of all B ciphertexts */
+/* the shape (ciphertexts per SM in a pass) of a launch of B ciphertexts: lvl02
+ * that of its first part, 1 where it runs one ciphertext per block; for
+ * CUFHEDB_FP64 and CUFHEDB_SPLIT32 on the CUDA cores, which run one ciphertext
+ * per block, the table's choice */
 CUFHEDB_API int cufhedb_launch_shape(cufhedb_ctx *ctx, int level, int precision, int B, int *shape);
 /* the stage-1 layout a CUFHEDB_SPLIT32 launch of B ciphertexts would use now:
  * *tensor_core_stage1 = 1 (tensor cores) or 0 (CUDA cores) */

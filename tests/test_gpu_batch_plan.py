@@ -93,6 +93,18 @@ def test_lvl02_runs_of_skipped_cmuxes(lvl2_engines, rows):
     assert torch.equal(*outs)
 
 
+def test_lvl02_launch_shape_is_the_shape_of_the_launch(lvl2_engines):
+    """untuned: the plan for a B200's times; a forced shape up to six ciphertexts per
+    SM; one ciphertext per block above"""
+    from cufhedb_b200 import FP64
+    S = lvl2_engines[0].num_sms
+    shape = lambda e, B: e.launch_shape(2, FP64, B)
+    assert [shape(lvl2_engines[0], B) for B in (1, S, S + 1, 2 * S, 2 * S + 1, 3 * S)] == [1, 1, 2, 2, 3, 3]
+    for k, e in enumerate(lvl2_engines[1:], 1):
+        assert [shape(e, B) for B in (1, 3 * S, 6 * S)] == [k] * 3
+    assert all(shape(e, B) == 1 for e in lvl2_engines for B in (6 * S + 1, 16384))
+
+
 def test_one_row_bootstraps_in_place(lvl2_engines):
     """the output over the row that it is made from, whose last CMuxes (or all) are
     skipped: no barrier stands between them and the output"""
