@@ -20,7 +20,7 @@ namespace cfdb {
 // scalar form with the paired form's roundings.  The compiler fuses a packed
 // product into the packed addition or subtraction that takes it (the first
 // operand's product where both are products), so the fused forms are written
-// out here; the tests compare whole bootstraps of both kernels word for word.
+// out here; cufhedb_selftest_split_transforms compares both forms bit for bit.
 // a * conj(c + i s)
 __device__ __forceinline__ float2 fmulc_t(float2 a, float c, float s)
 {

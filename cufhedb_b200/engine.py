@@ -393,6 +393,13 @@ class Engine:
         when the expired wait was recorded and reported, as it should be)"""
         return self.lib.cufhedb_selftest_wait_timeout(self.ctx, polls)
 
+    def selftest_split_transforms(self, seed: int = 1, blocks: int = 1024):
+        """how many values of the split path's block transforms differ from the
+        one-warp forms: (forward, inverse)"""
+        f, i = C.c_int(0), C.c_int(0)
+        check(self.lib.cufhedb_selftest_split_transforms(self.ctx, seed, blocks, C.byref(f), C.byref(i)))
+        return f.value, i.value
+
     ARC_OPS = {"gt": 0, "lt": 1, "eq": 2, "lt_strict": 3}
 
     def arc_compare(self, op: str, trlwe_dev, trgsw_prepared, out_dev, digits: int, precision=_lib.FP64,

@@ -385,6 +385,12 @@ CUFHEDB_API int cufhedb_compare_host_multi(cufhedb_ctx *const *ctxs, int nctx, i
  * cufhedb_sync reports after each: CUFHEDB_ERR_DEVICE with the wait's code when
  * both do; the context stays usable afterwards. */
 CUFHEDB_API int cufhedb_selftest_wait_timeout(cufhedb_ctx *ctx, uint32_t polls);
+/* Self-test of the split path's transforms (no counterpart in the reference): the
+ * forms that a block of warps runs against the one-warp forms of the
+ * tensor-core kernel on `blocks` (1 .. 65,536) random polynomials; how many of the
+ * 1,024 values (forward) and words (inverse) of each differ: none should. */
+CUFHEDB_API int cufhedb_selftest_split_transforms(cufhedb_ctx *ctx, uint32_t seed, int blocks, int *forward_differ,
+                                                  int *inverse_differ);
 
 /* ---- launch-shape autotuner --------------------------------------------------- */
 /* Launch shapes are ciphertexts per SM in a pass: lvl01 7, 8 and 4, lvl02 3, 2
@@ -399,7 +405,8 @@ CUFHEDB_API int cufhedb_selftest_wait_timeout(cufhedb_ctx *ctx, uint32_t polls);
  * next choice: CUFHEDB_SPLIT32 launches pick the layout of the first transform
  * step, on the CUDA cores or on the tensor cores (the CUFHEDB_SPLIT32_TC
  * kernel), by the same rule over both tables once both are measured, ties to
- * the CUDA cores.  The results are the same words in every shape.  No
+ * the CUDA cores.  The results are the same words in every shape of a
+ * layout (the tensor-core one rounds its first step differently).  No
  * counterpart in the reference, which runs one ciphertext per launch.  The
  * tuning calls are synchronous; call them outside stream capture. */
 /* times one full pass of each lvl01 shape for `precision` (uniform random lvl0

@@ -135,6 +135,15 @@ def test_one_row_bootstraps_in_place(lvl2_engines):
             assert torch.equal(buf, want)
 
 
+def test_split_block_transforms_equal_the_one_warp_forms():
+    """the packed one-warp transforms and the block's, bit for bit: both are the same
+    operations with the same roundings"""
+    from cufhedb_b200 import Engine
+    with Engine(0) as eng:
+        for seed in (1, 2):
+            assert eng.selftest_split_transforms(seed, 4096) == (0, 0)
+
+
 def _inputs(B):
     """uniform lvl0 words, with mask words that round to rotations 0 and N and
     an all-zero row among them"""
