@@ -328,7 +328,7 @@ struct PlainPath : SplitPath {
             twiddles(x, tm + 32, c);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                // pmul_t by conj(twist) / 512 (the scale is a power of two)
+                // times conj(twist) / 512 (the scale is a power of two)
                 const V a = v[8 * c + k], t = entry(x, k);
                 const float cs = t.x * (1.0f / 512.0f), sn = -t.y * (1.0f / 512.0f);
                 const float yr = fmaf(a.x, cs, -__fmul_rn(a.y, sn)), yi = fmaf(a.x, sn, __fmul_rn(a.y, cs));

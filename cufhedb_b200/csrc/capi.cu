@@ -110,16 +110,11 @@ void build_tables_f(const Fft512Tables &D, Fft512TablesF &F)
     for (int i = 0; i < 512; ++i) {
         P.tw512[i] = make_float2((float)D.tw512[i].x, (float)D.tw512[i].y);
         P.twist[i] = make_float2((float)D.twist[i].x, (float)D.twist[i].y);
-        P.tw512p[i] = dup(D.tw512[i].x, D.tw512[i].y);
-        P.untwistp[i] = dup(D.twist[i].x / 512.0, -D.twist[i].y / 512.0);
         const double2 t = cx(D.tw512[i], D.twist[i % 32]);   // W^{m1 q2} w^{m1}, m1 = i % 32
         Q.tw512w[i] = make_float2((float)t.x, (float)t.y);
         Q.tw512u[i] = dup(t.x / 512.0, t.y / 512.0);
     }
-    for (int j = 0; j < 16; ++j) {
-        P.w32[j] = make_float2((float)D.w32[j].x, (float)D.w32[j].y);
-        P.w32p[j] = Q.w32p[j] = dup(D.w32[j].x, D.w32[j].y);
-    }
+    for (int j = 0; j < 16; ++j) P.w32p[j] = Q.w32p[j] = dup(D.w32[j].x, D.w32[j].y);
     build_stage1_b(F.tc_b[0], F.tc_b[1]);
 }
 

@@ -9,15 +9,11 @@
 
 namespace cfdb {
 
-// Tables of the FP32 transforms.  The plain set: the twist, the stage-1 and
-// radix-2 twiddles as (c, s), and for the paired inverse the same with each
-// cosine and sine duplicated (c, c, s, s) plus the untwist (conj(twist) / 512).
+// Tables of the FP32 transforms.  The plain set (external products): the stage-1
+// twiddles and the twist as (c, s), the radix-2 twiddles (c, c, s, s).
 struct Fft512TablesPlain {
     float2 tw512[512];
     float2 twist[512];
-    float2 w32[16];
-    float4 tw512p[512];
-    float4 untwistp[512];   // conj(twist) / 512: inverse untwist and scaling in one product
     float4 w32p[16];
 };
 // The folded set: the lane's part of the twist rides on the forward stage-1
@@ -29,8 +25,8 @@ struct Fft512TablesFold {
     float4 tw512u[512];   // tw512u[k * 32 + m1] = W^{m1 k} w^{m1} / 512 (used conjugated)
     float4 w32p[16];
 };
-// both sets, as the context keeps them in global memory; a kernel copies the
-// set it uses into shared memory.  tc_b: the two FP16 limbs of the constant
+// both sets, as the context keeps them in global memory; a kernel copies what it
+// uses of one into tensor or shared memory.  tc_b: the two FP16 limbs of the constant
 // matrix of the tensor-core stage 1 (tc_stage1.cuh), hi then lo.
 struct Fft512TablesF {
     Fft512TablesPlain plain;
@@ -228,13 +224,7 @@ __device__ __forceinline__ unsigned long long f2(unsigned long long a, unsigned 
 
 __device__ __forceinline__ CP padd(CP a, CP b) { return CP{a2(a.re, b.re), a2(a.im, b.im)}; }
 __device__ __forceinline__ CP psub(CP a, CP b) { return CP{s2(a.re, b.re), s2(a.im, b.im)}; }
-// a * (c + i s) for a twiddle stored (c, c, s, s)
-__device__ __forceinline__ CP pmul_t(CP a, float4 w)
-{
-    const unsigned long long C = pk2(w.x, w.y), S = pk2(w.z, w.w);
-    return CP{s2(m2(a.re, C), m2(a.im, S)), f2(a.re, S, m2(a.im, C))};
-}
-// a * conj(c + i s)
+// a * conj(c + i s) for a twiddle stored (c, c, s, s)
 __device__ __forceinline__ CP pmulc_t(CP a, float4 w)
 {
     const unsigned long long C = pk2(w.x, w.y), S = pk2(w.z, w.w);
@@ -320,13 +310,11 @@ __device__ __forceinline__ void pdft16(CP v[16])
 // inverse transform of two polynomials at once (the forward steps in reverse
 // with conjugate twiddles);
 // xp: this warp's FFT512_XP 8-byte entries, through which the real and the
-// imaginary parts are transposed one after the other.  Output v[m2] =
-// 512 z_{lane + 32 m2} (multiply by untwistp to finish); with FOLD the stage-1
-// twiddles (tw512u) also carry conj(w^{lane}) / 512, so the output is
-// z_{lane + 32 m2} w^{32 m2}... times the rest of the twist only, which
+// imaginary parts are transposed one after the other.  The stage-1 twiddles
+// (tw512u) also carry conj(w^{lane}) / 512, so the output v[m2] is
+// z_{lane + 32 m2} times the rest of the twist only, which
 // untwist_m2 removes with compile-time constants instead of a table read.
-template <bool FOLD, class TT>
-__device__ __forceinline__ void pfft512_inv(CP v[16], unsigned long long *xp, const TT &T, int lane)
+__device__ __forceinline__ void pfft512_inv(CP v[16], unsigned long long *xp, const Fft512TablesFold &T, int lane)
 {
     const int h = lane >> 4, q2 = lane & 15;
 #pragma unroll
@@ -351,28 +339,13 @@ __device__ __forceinline__ void pfft512_inv(CP v[16], unsigned long long *xp, co
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < 16; ++k) v[k].im = xp[xpf_index(lane, k)];
-    if constexpr (FOLD) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = pmulc_t(v[k], T.tw512u[k * 32 + lane]);
-    } else {
-#pragma unroll
-        for (int k = 1; k < 16; ++k) v[k] = pmulc_t(v[k], T.tw512p[k * 32 + lane]);
-    }
+    for (int k = 0; k < 16; ++k) v[k] = pmulc_t(v[k], T.tw512u[k * 32 + lane]);
     pdft16<-1>(v);
 }
 
 // a * conj(e^{2 pi i m2 / 64}) = a * conj(w^{32 m2}): the per-register part of
 // the untwist left after pfft512_inv (compile-time constants once unrolled)
-__device__ __forceinline__ float2 untwist_m2(float2 a, int m2)
-{
-    constexpr float C[16] = {1.000000000e+00f, 9.951847267e-01f, 9.807852804e-01f, 9.569403357e-01f,
-                             9.238795325e-01f, 8.819212643e-01f, 8.314696123e-01f, 7.730104534e-01f,
-                             7.071067812e-01f, 6.343932842e-01f, 5.555702330e-01f, 4.713967368e-01f,
-                             3.826834324e-01f, 2.902846773e-01f, 1.950903220e-01f, 9.801714033e-02f};
-    if (m2 == 0) return a;
-    const float c = C[m2], sn = C[16 - m2];
-    return make_float2(fmaf(a.x, c, a.y * sn), fmaf(a.y, c, -a.x * sn));
-}
 __device__ __forceinline__ CP untwist_m2(CP a, int m2)
 {
     constexpr float C[16] = {1.000000000e+00f, 9.951847267e-01f, 9.807852804e-01f, 9.569403357e-01f,
@@ -382,6 +355,5 @@ __device__ __forceinline__ CP untwist_m2(CP a, int m2)
     if (m2 == 0) return a;
     return pmulc_t(a, make_float4(C[m2], C[m2], C[16 - m2], C[16 - m2]));
 }
-
 
 }  // namespace cfdb

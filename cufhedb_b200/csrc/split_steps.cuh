@@ -57,7 +57,7 @@ __device__ __forceinline__ uint32_t hi_term(float h)
 __device__ __forceinline__ void add_inverse_split(uint32_t *poly, CP f[16], unsigned long long *xp, int lane,
                                                   const Fft512TablesFold &T)
 {
-    pfft512_inv<true>(f, xp, T, lane);
+    pfft512_inv(f, xp, T, lane);
 #pragma unroll
     for (int m2 = 0; m2 < 16; ++m2) {
         const int m = lane + 32 * m2;
