@@ -47,7 +47,7 @@ WORKLOAD = ("1,024 lvl1 HomNAND gate bootstraps (IKS10 + PBS01 each) over unifor
             "TFHEpp 128-bit params (n=672, N=1024, l=3, Bg=2^6, IKS10 basebit 10 t 2)")
 # DRAM bytes (read + write) of one 1,024-ciphertext PBS launch, from the ncu
 # captures summarised under profiles/ (pbs01_*_batch1024.md)
-TRAFFIC = {"split32": 93_320_000 + 6_280_000, "fp64": 148_770_000 + 6_980_000}
+TRAFFIC = {"split32": 96_900_000 + 4_800_000, "fp64": 129_510_000 + 7_500_000}
 
 
 def parse(argv=None):

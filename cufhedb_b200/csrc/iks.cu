@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(NT) iks_kernel(IksArgs a)
 //   lvl20   1: 0.395 -> 0.026;  148: 1.08 -> 0.262;  592: 1.11 -> 0.768;
 //     750: 1.14 -> 1.05;  850: 1.16 -> 1.18;  1,100: 1.27 -> 1.49;  1,184: 1.30 -> 1.33;
 //     1,185: 2.33 -> 1.40;  1,850: 2.45 -> 2.37;  1,900: 2.47 -> 2.56
-//   lvl21   1: 3.42 -> 0.037;  148: 2.55 -> 0.58;  511: 2.22 -> 1.94
+//   lvl21   1: 3.38 -> 0.026;  148: 2.49 -> 0.60;  511: 2.26 -> 2.10
 struct GatherRule {
     double few, wave, tail;   // ciphertexts per SM
 };
@@ -259,8 +259,9 @@ cudaError_t launch_gather(const IksArgs &a, const GatherRule &rule, cudaStream_t
 // part of the key, staging those 8 words of every key row in shared memory, and
 // each thread, one ciphertext, subtracts the staged words of the rows its digits
 // select.  Integer sums modulo 2^32: the parts add up to the gather's words.
-// Bound by the shared-memory reads (two of 16 bytes per digit, a wavefront per
-// quarter-warp: 2.4 ms per 1,024) and, per tile, by the staging (about 0.3 ms):
+// Bound by the L1 data pipe (93 % busy at 200 and at 1,024), which serves the
+// shared-memory reads (two of 16 bytes per digit, a wavefront per quarter-warp: 2.4 ms
+// per 1,024) and, per tile, the staging (about 0.3 ms):
 // so 512 ciphertexts share a tile where there are more than 256, and warps past
 // the batch only stage.  The staged rows are padded to 48 bytes, so the eight
 // digit values of a quarter-warp's 16-byte reads fall in eight distinct bank

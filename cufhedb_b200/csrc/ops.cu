@@ -248,9 +248,12 @@ struct Ops {
 
     // equal on both orders at once: NOT MSB(c1 - c2) and NOT MSB(c2 - c1) as one
     // chain over 2 B rows, then HomAND.  A chain lasts as long for one row as for
-    // a full pass (a 16-bit one 31 ms up to 148 rows), so below EQ_JOINT rows one
-    // chain of twice the rows takes little more than either of two; above, the
-    // passes are full anyway and the scratch stays at one chain's.
+    // 148, so below EQ_JOINT rows one chain of twice the rows takes less than two;
+    // at the line the gain has shrunk to a few per cent (the batches fill the GPU
+    // anyway) and above it the scratch stays at one chain's.  ms, two chains -> one,
+    // split: lvl1 4 bits 1: 5.98 -> 4.00, 148: 6.10 -> 5.16, 444: 12.6 -> 12.3, 1,024:
+    // 27.4 -> 27.0; lvl2 16 bits 1: 62.9 -> 32.2, 148: 63.4 -> 57.8, 500: 221 -> 191,
+    // 1,024: 380 -> 367; FP64 alike.
     static constexpr int EQ_JOINT = 1024;
     template <int LVL, typename T>
     int equal_joint(const T *a, const T *b, uint32_t *out, uint32_t pb, bool arith)
